@@ -779,8 +779,20 @@ struct EngineChunk {
 // static slice may belong to a CTA that is not resident yet.  (Measured on
 // B200: the static form is 3-4% faster on the Q path's short launches and
 // 0.5% slower on the benchmark's long ones, so each plan gets its form.)
-template <class Epi, int PREC, bool kStatic>
-__global__ void __launch_bounds__(kEngineThreads, EngineMinBlocks<Epi>::value) engine_kernel(EngineArgs a, Epi epi) {
+//
+// kWide (host-chosen, plans of at most one tile per warp at two CTAs per SM):
+// a launch then lasts as long as one tile's chain, and more warps per SM
+// cannot shorten it; two CTAs per SM leave 128 registers per thread, so
+// eight nonzeros per lane are in flight and nothing spills.  (Measured on
+// B200, us per iteration with the three-CTA form / this one: n = 2000 33.3 /
+// 27.9, n = 3000 with a CSR Q 34.1 / 30.3, n = 100k 34.7 / 29.2.  Past one
+// tile per warp the third CTA hides more latency: n = 2M 262 / 269.)
+constexpr int kWideBlocks = 2;
+constexpr int kWideChunk = 8;
+template <class Epi, int PREC, bool kStatic, bool kWide>
+__global__ void __launch_bounds__(kEngineThreads, kWide ? kWideBlocks : EngineMinBlocks<Epi>::value)
+    engine_kernel(EngineArgs a, Epi epi) {
+  constexpr int kCh = kWide ? kWideChunk : EngineChunk<Epi>::value;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   WarpSmem* s_ws = reinterpret_cast<WarpSmem*>(smem_raw);
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -803,7 +815,7 @@ __global__ void __launch_bounds__(kEngineThreads, EngineMinBlocks<Epi>::value) e
     }
     while (base < ntasks) {
       for (int q = 0; q < kGrab && base + q < ntasks; ++q)
-        process_warp_tile<Epi, PREC, false, EngineChunk<Epi>::value>(a, epi, base + q, ws);
+        process_warp_tile<Epi, PREC, false, kCh>(a, epi, base + q, ws);
       int next = ntasks;
       if (dyn && lane == 0) next = nstat + atomicAdd(a.pv.task_ctr, kGrab);
       base = __shfl_sync(0xffffffffu, next, 0);
@@ -823,7 +835,7 @@ __global__ void __launch_bounds__(kEngineThreads, EngineMinBlocks<Epi>::value) e
           pf = __shfl_sync(0xffffffffu, next, 0);
           pf = pf < ntasks ? pf : -1;
         }
-        process_warp_tile<Epi, PREC, false, EngineChunk<Epi>::value>(a, epi, base + q, ws, pf);
+        process_warp_tile<Epi, PREC, false, kCh>(a, epi, base + q, ws, pf);
       }
       if (!HPR_ENGINE_EARLYGRAB && lane == 0) next = atomicAdd(a.pv.task_ctr, kGrab);
       base = __shfl_sync(0xffffffffu, next, 0);

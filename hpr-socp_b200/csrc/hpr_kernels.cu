@@ -210,15 +210,17 @@ namespace {
 
 // Persistent grid size of one engine instantiation (resident CTAs per SM x
 // SMs), computed once.
-template <class Epi, int PREC, bool kStatic>
+template <class Epi, int PREC, bool kStatic, bool kWide>
 int engine_grid(int* smem_bytes) {
   static std::once_flag once;
   static int grid = 1;
   constexpr int dyn = kEngineSmem;
   *smem_bytes = dyn;
   std::call_once(once, [] {
-    auto k = engine_kernel<Epi, PREC, kStatic>;
+    auto k = engine_kernel<Epi, PREC, kStatic, kWide>;
     cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn);
+    // (the kWide form keeps the other form's carveout: an SM drains before it
+    // changes its carveout, which cost the Q path's mixed launches 3.4 of 136 us)
     const int carve = HPR_ENGINE_CARVEOUT >= 0 ? (int)(HPR_ENGINE_CARVEOUT)
                                                : engine_carveout(EngineMinBlocks<Epi>::value);
     cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, carve);
@@ -233,10 +235,10 @@ int engine_grid(int* smem_bytes) {
 
 // One warp per tile at most: a small problem occupies only the SMs it needs,
 // so other streams (other contexts of a serving process) run beside it.
-template <class Epi, int PREC, bool kStatic>
+template <class Epi, int PREC, bool kStatic, bool kWide>
 void launch_engine_form(Ctx* c, int nt, const EngineArgs& a, const Epi& epi) {
   int dyn = 0;
-  const int full = engine_grid<Epi, PREC, kStatic>(&dyn);
+  const int full = engine_grid<Epi, PREC, kStatic, kWide>(&dyn);
   const int g = std::max(1, std::min(full, (nt + kWarpsPerCta - 1) / kWarpsPerCta));
 #if HPR_ENGINE_PDL
   // programmatic dependent launch: the kernel may be scheduled while the
@@ -252,10 +254,23 @@ void launch_engine_form(Ctx* c, int nt, const EngineArgs& a, const Epi& epi) {
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  cudaLaunchKernelEx(&cfg, engine_kernel<Epi, PREC, kStatic>, a, epi);
+  cudaLaunchKernelEx(&cfg, engine_kernel<Epi, PREC, kStatic, kWide>, a, epi);
 #else
-  engine_kernel<Epi, PREC, kStatic><<<g, kEngineThreads, dyn, c->stream>>>(a, epi);
+  engine_kernel<Epi, PREC, kStatic, kWide><<<g, kEngineThreads, dyn, c->stream>>>(a, epi);
 #endif
+}
+
+// tiles of one wave of the kWide form: one per warp, two CTAs per SM
+int engine_wide_tiles() {
+  static std::once_flag once;
+  static int tiles = 0;
+  std::call_once(once, [] {
+    int dev = 0, sms = 148;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    tiles = kWideBlocks * kWarpsPerCta * sms;
+  });
+  return tiles;
 }
 
 // Plans without split cones take their first tiles by warp index
@@ -263,8 +278,14 @@ void launch_engine_form(Ctx* c, int nt, const EngineArgs& a, const Epi& epi) {
 // counter.
 template <class Epi, int PREC>
 void launch_engine_prec(Ctx* c, int nt, const EngineArgs& a, const Epi& epi) {
-  if (a.pv.nbig == 0) launch_engine_form<Epi, PREC, true>(c, nt, a, epi);
-  else launch_engine_form<Epi, PREC, false>(c, nt, a, epi);
+  const bool wide = nt <= engine_wide_tiles();
+  if (a.pv.nbig == 0) {
+    if (wide) launch_engine_form<Epi, PREC, true, true>(c, nt, a, epi);
+    else launch_engine_form<Epi, PREC, true, false>(c, nt, a, epi);
+  } else {
+    if (wide) launch_engine_form<Epi, PREC, false, true>(c, nt, a, epi);
+    else launch_engine_form<Epi, PREC, false, false>(c, nt, a, epi);
+  }
 }
 
 template <class Epi>
