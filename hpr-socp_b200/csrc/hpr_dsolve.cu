@@ -899,9 +899,8 @@ __global__ void __launch_bounds__(kDThreads, 1)
 bool dsolve_eligible(const Ctx* c, const hpr_params* P) {
   if (P->precision != HPR_PREC_FP64 || P->auto_save) return false;
   if (c->q_kind == HPR_Q_DIAG_LOWRANK || c->q_kind == HPR_Q_OPERATOR) return false;
-  auto fits = [](const Plan& p) { return (int64_t)p.tasks.size() <= kFusedMaxTiles; };
-  if (!fits(c->planX) || !fits(c->planY)) return false;
-  if (c->has_q && !fits(c->planQ)) return false;
+  if (!one_cta_plan(c->planX) || !one_cta_plan(c->planY)) return false;
+  if (c->has_q && !one_cta_plan(c->planQ)) return false;
   return kEngineSmem <= 48 * 1024;
 }
 

@@ -287,6 +287,18 @@ __device__ __forceinline__ void prefetch_l2(const void* p, int64_t bytes) {
   asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(b), "r"((uint32_t)(e - b)) : "memory");
 }
 
+// shared-memory accesses by 32-bit address (through a generic pointer that the
+// compiler cannot place, each costs more instructions and latency)
+__device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ double lds_f64(uint32_t a) {
+  double v;
+  asm volatile("ld.shared.f64 %0, [%1];" : "=d"(v) : "r"(a) : "memory");
+  return v;
+}
+__device__ __forceinline__ void sts_f64(uint32_t a, double v) {
+  asm volatile("st.shared.f64 [%0], %1;" ::"r"(a), "d"(v) : "memory");
+}
+
 struct WarpSmem {
   double acc[kRowCap + 32];  // row sums by non-empty ordinal, then raw cone values by row;
                              // from kRowCap: each lane's continuation of an earlier run's row
@@ -579,7 +591,8 @@ __device__ __forceinline__ void prefetch_tile(const EngineArgs& a, const Epi& ep
 // CH (U): nonzeros per lane per step.
 // pf_next >= 0: the warp's next tile, prefetched to L2 after this tile's
 // gathers.
-template <class Epi, int PREC, bool kCoherent = false, int CH = kChunk>
+// kRows: the plan may hold tiles in row mode.
+template <class Epi, int PREC, bool kCoherent = false, int CH = kChunk, bool kRows = true>
 __device__ void process_warp_tile(const EngineArgs& a, Epi& epi, int tix, WarpSmem& ws, int pf_next = -1) {
   constexpr int U = CH;
   const int lane = threadIdx.x & 31;
@@ -601,12 +614,15 @@ __device__ void process_warp_tile(const EngineArgs& a, Epi& epi, int tix, WarpSm
   // for nonzeros in flight
   const int nnz = tp->nze - tp->nzb;
   const uint64_t desc = a.pv.desc[(int64_t)tix * 32 + lane];
-  const int R = (nnz + 31) >> 5;
+  const TileRun* rp = a.pv.runs + tix;
+  const bool rows = kRows && rp->r0 >= 0;  // row mode: the lane's rows, one after the other
+  int R = rows ? rp->r0 : (nnz + 31) >> 5;
   int my = nnz - lane * R;
-  my = my < 0 ? 0 : (my > R ? R : my);
+  my = rows ? (int)(desc & 0xffff) : (my < 0 ? 0 : (my > R ? R : my));
   const uint64_t pol = HPR_ENGINE_STREAM == 2 ? l2_evict_first_policy() : 0;
-  const uint32_t heads = (uint32_t)desc;
+  const uint32_t heads = rows ? 0u : (uint32_t)desc;
   const int j0 = (int)(desc >> kDescOrdShift);
+  double acc0 = 0.0, acc1 = 0.0;  // sums of rows rb + lane and rb + lane + 32
   Vals<Epi::kSlots> v0, v1;
   if (HPR_ENGINE_PREFETCH && tp->kind != TASK_LONG_PART) {
     const Task t = *tp;
@@ -617,11 +633,12 @@ __device__ void process_warp_tile(const EngineArgs& a, Epi& epi, int tix, WarpSm
   }
 
   // ---- 1. products, added per lane in column order
-  const int64_t base = (int64_t)a.pv.runs[tix].sbase + lane;
+  int64_t base = (int64_t)rp->sbase + lane;
   double s = 0.0;
-  int cur = j0;                                  // non-empty ordinal of the next row to start
-  double* close = ws.acc + kRowCap + lane;       // where the segment being summed goes
-  {
+  const uint32_t acc = smem_addr(ws.acc);
+  uint32_t next = acc + 8 * j0;                  // slot of the next row to start (by non-empty ordinal)
+  uint32_t close = acc + 8 * (kRowCap + lane);   // where the segment being summed goes
+  for (int h = 0;; ++h) {
     // one base address per array and step; the U loads of a step sit at
     // fixed offsets from it
     auto load_step = [&](int k0, int32_t* cc, double* vv) {
@@ -661,6 +678,7 @@ __device__ void process_warp_tile(const EngineArgs& a, Epi& epi, int tix, WarpSm
         }
       }
       if (!HPR_ENGINE_PIPE && k0 + U < R) load_step(k0 + U, ncols, nvals);
+      const uint32_t hb = heads >> (k0 & 31);
 #pragma unroll
       for (int u = 0; u < U; ++u) {
         // a row starts here: close the previous segment.  A predicated
@@ -670,11 +688,11 @@ __device__ void process_warp_tile(const EngineArgs& a, Epi& epi, int tix, WarpSm
         // 4.4M-nonzero Q path 147 / 136, n = 3000 with a CSR Q 43.9 / 34.1,
         // n = 400 in one CTA 14.5 / 12.2).  Descriptor bits beyond the run
         // are 0 and so are its products.
-        const bool head = (heads >> (k0 + u)) & 1u;
+        const bool head = (hb >> u) & 1u;
         if (head) {
-          *close = s;
-          close = ws.acc + cur;
-          ++cur;
+          sts_f64(close, s);
+          close = next;
+          next += 8;
         }
         s = (head ? 0.0 : s) + p[u];
       }
@@ -684,9 +702,20 @@ __device__ void process_warp_tile(const EngineArgs& a, Epi& epi, int tix, WarpSm
         vals[u] = nvals[u];
       }
     }
+    if constexpr (!kRows) break;
+    if (!rows) break;
+    if (h > 0 || rp->r1 == 0) {
+      (h > 0 ? acc1 : acc0) = s;
+      break;
+    }
+    acc0 = s;
+    s = 0.0;
+    base += 32 * (int64_t)R;
+    R = rp->r1;
+    my = (int)((desc >> 16) & 0xffff);
   }
-  if (my > 0) *close = s;
-  const double cont = my > 0 ? ws.acc[kRowCap + lane] : 0.0;
+  if (!rows && my > 0) sts_f64(close, s);
+  const double cont = !rows && my > 0 ? lds_f64(acc + 8 * (kRowCap + lane)) : 0.0;
 
   if (HPR_ENGINE_L2PF >= 2 && pf_next >= 0) prefetch_tile<Epi, PREC>(a, epi, pf_next);
   const Task t = *tp;
@@ -709,7 +738,7 @@ __device__ void process_warp_tile(const EngineArgs& a, Epi& epi, int tix, WarpSm
 
   // ---- 2. continuations: segmented scan over the lanes, then added to the
   // row's head segment
-  {
+  if (!rows) {
     const bool has_cont = my > 0 && !(heads & 1u);
     const int key = has_cont ? j0 - 1 : -2 - lane;
     double v = has_cont ? cont : 0.0;
@@ -724,19 +753,18 @@ __device__ void process_warp_tile(const EngineArgs& a, Epi& epi, int tix, WarpSm
     }
     const int nk = __shfl_down_sync(0xffffffffu, key, 1);
     __syncwarp();  // head segments are in ws.acc
-    if (has_cont && (lane == 31 || nk != key)) ws.acc[key] = ws.acc[key] + v;
+    if (has_cont && (lane == 31 || nk != key)) sts_f64(acc + 8 * key, lds_f64(acc + 8 * key) + v);
     __syncwarp();
   }
 
   // ---- 3. row sums to the owning lanes (empty rows sum to zero)
-  double acc0 = 0.0, acc1 = 0.0;
-  {
+  if (!rows) {
     const unsigned lt = (1u << lane) - 1u;
-    const uint64_t ne = a.pv.runs[tix].nonempty;
+    const uint64_t ne = rp->nonempty;
     const unsigned b0 = (unsigned)(ne & 0xffffffffull);
     const unsigned b1 = (unsigned)(ne >> 32);
-    if ((b0 >> lane) & 1u) acc0 = ws.acc[__popc(b0 & lt)];
-    if (kTwoRows && ((b1 >> lane) & 1u)) acc1 = ws.acc[__popc(b0) + __popc(b1 & lt)];
+    if ((b0 >> lane) & 1u) acc0 = lds_f64(acc + 8 * __popc(b0 & lt));
+    if (kTwoRows && ((b1 >> lane) & 1u)) acc1 = lds_f64(acc + 8 * (__popc(b0) + __popc(b1 & lt)));
     __syncwarp();
   }
 
@@ -780,7 +808,8 @@ struct EngineChunk {
 // B200: the static form is 3-4% faster on the Q path's short launches and
 // 0.5% slower on the benchmark's long ones, so each plan gets its form.)
 //
-// kWide (host-chosen, plans of at most one tile per warp at two CTAs per SM):
+// kWide (host-chosen, plans of at most one tile per warp at two CTAs per SM;
+// plans with row-mode tiles are always of that size):
 // a launch then lasts as long as one tile's chain, and more warps per SM
 // cannot shorten it; two CTAs per SM leave 128 registers per thread, so
 // eight nonzeros per lane are in flight and nothing spills.  (Measured on
@@ -815,7 +844,7 @@ __global__ void __launch_bounds__(kEngineThreads, kWide ? kWideBlocks : EngineMi
     }
     while (base < ntasks) {
       for (int q = 0; q < kGrab && base + q < ntasks; ++q)
-        process_warp_tile<Epi, PREC, false, kCh>(a, epi, base + q, ws);
+        process_warp_tile<Epi, PREC, false, kCh, kWide>(a, epi, base + q, ws);
       int next = ntasks;
       if (dyn && lane == 0) next = nstat + atomicAdd(a.pv.task_ctr, kGrab);
       base = __shfl_sync(0xffffffffu, next, 0);
@@ -835,7 +864,7 @@ __global__ void __launch_bounds__(kEngineThreads, kWide ? kWideBlocks : EngineMi
           pf = __shfl_sync(0xffffffffu, next, 0);
           pf = pf < ntasks ? pf : -1;
         }
-        process_warp_tile<Epi, PREC, false, kCh>(a, epi, base + q, ws, pf);
+        process_warp_tile<Epi, PREC, false, kCh, kWide>(a, epi, base + q, ws, pf);
       }
       if (!HPR_ENGINE_EARLYGRAB && lane == 0) next = atomicAdd(a.pv.task_ctr, kGrab);
       base = __shfl_sync(0xffffffffu, next, 0);

@@ -110,7 +110,8 @@ PlanView view_of(const Plan& p, const int32_t* cone_start) {
 // ---------------------------------------------------------------------------
 namespace {
 template <class T>
-__global__ void tile_layout_kernel(const Task* __restrict__ tasks, const TileRun* __restrict__ runs, int ntasks,
+__global__ void tile_layout_kernel(const Task* __restrict__ tasks, const TileRun* __restrict__ runs,
+                                   const uint64_t* __restrict__ desc, int ntasks,
                                    const int32_t* __restrict__ col, const T* __restrict__ val,
                                    int32_t* __restrict__ tcol, T* __restrict__ tval) {
   const int lane = threadIdx.x & 31;
@@ -121,6 +122,27 @@ __global__ void tile_layout_kernel(const Task* __restrict__ tasks, const TileRun
     const int32_t nnz = t.nze - t.nzb;
     const int32_t R = (nnz + 31) / 32;
     const int64_t sb = runs[ti].sbase;
+    if (runs[ti].r0 >= 0) {
+      // row mode: a lane's rows start at the sum of the rows before them
+      const uint64_t d = desc[ti * 32 + lane];
+      int32_t start = t.nzb;
+      for (int h = 0; h < 2; ++h) {
+        const int32_t len = (int32_t)((d >> (16 * h)) & 0xffff), steps = h ? runs[ti].r1 : runs[ti].r0;
+        int32_t inc = len;
+        for (int o = 1; o < 32; o <<= 1) {
+          const int32_t v = __shfl_up_sync(0xffffffffu, inc, o);
+          if (lane >= o) inc += v;
+        }
+        const int64_t s0 = sb + 32 * (int64_t)(h ? runs[ti].r0 : 0) + lane;
+        for (int32_t k = 0; k < steps; ++k) {
+          const int32_t e = start + inc - len + k;
+          if (tcol) tcol[s0 + 32 * k] = k < len ? col[e] : 0;
+          tval[s0 + 32 * k] = k < len ? val[e] : T(0.0f);
+        }
+        start += __shfl_sync(0xffffffffu, inc, 31);
+      }
+      continue;
+    }
     for (int32_t k = 0; k < R; ++k) {
       const int32_t e = lane * R + k;  // element k of this lane's run
       const int64_t d = sb + 32 * (int64_t)k + lane;
@@ -140,7 +162,7 @@ int tile_layout(Ctx* c, const Plan& p, const int32_t* col, const T* val, int32_t
   const int nt = (int)p.tasks.size();
   if (nt == 0) return HPR_OK;
   const int blocks = std::min(148 * 8, (nt + 7) / 8);
-  tile_layout_kernel<T><<<blocks, 256, 0, c->stream>>>(p.d_tasks, p.d_runs, nt, col, val, tcol, tval);
+  tile_layout_kernel<T><<<blocks, 256, 0, c->stream>>>(p.d_tasks, p.d_runs, p.d_desc, nt, col, val, tcol, tval);
   c->launches++;
   HPR_CUDA(c, cudaGetLastError());
   return HPR_OK;
@@ -525,10 +547,9 @@ int launch_fused_prec(Ctx* c, const FStage<E0>& s0, const FStage<E1>& s1, const 
 
 bool fused_eligible(const Ctx* c) {
   if (c->q_kind == HPR_Q_DIAG_LOWRANK || c->q_kind == HPR_Q_OPERATOR) return false;
-  auto fits = [](const Plan& p) { return (int64_t)p.tasks.size() <= kFusedMaxTiles; };
-  if (!fits(c->planX) || !fits(c->planY)) return false;
+  if (!one_cta_plan(c->planX) || !one_cta_plan(c->planY)) return false;
   // with Q the reduced-precision streams apply to A only; keep those unfused
-  if (c->has_q && (!fits(c->planQ) || c->precision != HPR_PREC_FP64)) return false;
+  if (c->has_q && (!one_cta_plan(c->planQ) || c->precision != HPR_PREC_FP64)) return false;
   return kEngineSmem <= kSmemOptinMax;
 }
 
@@ -626,6 +647,7 @@ int tune_trial(Ctx* c, int64_t k, bool full_last) {
 }  // namespace
 
 bool uses_fused_iterations(const Ctx* c) {
+  if (c->schedule != HPR_SCHEDULE_ENGINE && resident_eligible(c)) return true;
   if (!fused_eligible(c)) return false;
   const int mode = c->schedule != HPR_SCHEDULE_AUTO ? c->schedule : tune_lookup(c);
   return mode != HPR_SCHEDULE_ENGINE;
@@ -636,6 +658,13 @@ int run_iterations(Ctx* c, int64_t k, bool full_last) {
   int64_t l0 = c->launches;
   HPR_CUDA(c, cudaEventRecord(c->ev0, c->stream));
   int mode = HPR_SCHEDULE_ENGINE;
+  if (c->schedule != HPR_SCHEDULE_ENGINE && resident_eligible(c)) {
+    HPR_TRY(launch_resident(c, k, full_last));
+    HPR_CUDA(c, cudaEventRecord(c->ev1, c->stream));
+    c->inner += k;
+    c->last_launches = c->launches - l0;
+    return HPR_OK;
+  }
   if (fused_eligible(c)) {
     mode = c->schedule != HPR_SCHEDULE_AUTO ? c->schedule : tune_lookup(c);
     if (mode == HPR_SCHEDULE_AUTO) {
@@ -1213,8 +1242,7 @@ int launch_power_A(Ctx* c, int maxit, double tol, double* lam) {
     *lam = 0.0;
     return HPR_OK;
   }
-  auto small = [](const Plan& p) { return (int64_t)p.tasks.size() <= kFusedMaxTiles; };
-  if (small(c->planX) && small(c->planY) && kEngineSmem <= kSmemOptinMax) return power_fused_A(c, maxit, tol, lam);
+  if (one_cta_plan(c->planX) && one_cta_plan(c->planY) && kEngineSmem <= kSmemOptinMax) return power_fused_A(c, maxit, tol, lam);
   return power_two_pass_A(c, maxit, tol, lam);
 }
 

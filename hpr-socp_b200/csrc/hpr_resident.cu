@@ -1,0 +1,710 @@
+// hpr_resident.cu — whole batches of HPR iterations for problems that fit
+// the shared memory of one thread-block cluster.
+//
+// A small problem's half-step is a chain of dependent memory round trips (tile
+// record, columns, gathers, epilogue inputs, stores) and of instructions, not
+// bytes.  Measured on B200, us per iteration of a 150-iteration batch, before
+// (single-CTA kernel through L2 up to n = 400, else the multi-CTA engine) and
+// here: n = 61 5.7 / 3.7, n = 400 12.0 / 7.1, n = 800 22 / 10.6, the same with
+// a diagonal Q 25.6 / 14.4, n = 2000 27.6 / 14.7, n = 3000 with a general CSR
+// Q 30 / 14.8.  What is left is mostly the row sums' and cones' chains.
+// Here every CTA of one cluster copies its share of the matrices (columns as
+// 16 bits, values in FP64, in the engine's run layout) and the tile records
+// into shared memory once per batch and keeps a full copy of each gathered
+// vector (x_hat and y; w, w_bar, tempv and y_bar with Q) there, so the chain
+// of a half-step is shared-memory latency: the rows' epilogue inputs are
+// requested from L2 before the row sums and arrive behind them.  A row's new
+// value is stored into every CTA's copy (distributed shared memory), and one
+// cluster barrier ends the half-step.
+//
+// Tile t belongs to CTA t mod C and within it to warp (t / C) mod kResWarps.
+// Sums, projections and their order are the engine's (hpr_engine.cuh), so the
+// iterates are the engine's to the bit.
+#include <algorithm>
+#include <mutex>
+#include <set>
+
+#include "hpr_epilogues.cuh"
+
+namespace hpr {
+
+namespace {
+
+constexpr int kResWarps = 16;
+constexpr int kResThreads = kResWarps * 32;
+constexpr int kResMaxCtas = 16;
+constexpr int kResSmemMax = 226 * 1024;
+constexpr int kResUnroll = 4;  // nonzeros per lane per step
+
+__host__ __device__ inline int pad_steps(int n) { return (n + kResUnroll - 1) / kResUnroll * kResUnroll; }
+
+struct ResTile {
+  int32_t rb, nrows, nnz, soff;  // soff: first slot in this CTA's arrays
+  uint64_t nonempty;
+  int16_t kind, ncones;
+  int32_t cone, group, part;
+  int32_t r0, r1;
+};
+static_assert(sizeof(ResTile) == 48, "ResTile layout");
+
+// cone layout of a tile of whole cones: row of each row's cone head, first
+// row of each cone (+ end)
+struct ResCones {
+  uint8_t head[kRowCap];
+  uint8_t start[kRowCap + 4];
+};
+
+struct ResSide {
+  const Task* tasks;
+  const TileRun* runs;
+  const uint64_t* desc;
+  const int32_t* tcol;
+  const double* tval;
+  const int32_t* cone_start;
+  const BigCone* big;
+  double *raw, *cpart;
+  int32_t ntasks, nwork, nbig;  // tasks, tasks before the apply tiles, split cones
+  int32_t o_val, o_desc, o_tile, o_cone, o_col;  // byte offsets in shared memory
+};
+
+// One half-step: epilogue, matrix side, gathered vector and the vector the
+// next half-steps gather (shared-memory copies at byte offsets gin / gout;
+// the global vector is kept too).
+template <class E>
+struct RStage {
+  E e;
+  int side, gin, gout;
+  double* gglob;
+  int on;
+};
+
+struct ResArgs {
+  ResSide side[3];  // A', A, Q
+  int nsides;
+  const double* g0;  // vector gathered by the first half-step
+  int g0_off, g0_len;
+  int o_state, o_ws;
+  DevState* st;
+  int iters, full_last;
+};
+
+struct ResWs {
+  double acc[kRowCap + 32];  // as WarpSmem
+  double sq[kRowCap];        // squares of the raw cone values; a cone's norm at its first row
+};
+
+__device__ __forceinline__ uint32_t cluster_rank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ uint32_t cluster_size() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
+  return r;
+}
+
+// All CTAs of the cluster (a CTA barrier when the cluster is one CTA); the
+// writes before it, local, remote and global, are visible after it.
+__device__ __forceinline__ void res_sync(uint32_t C) {
+  if (C == 1) {
+    __syncthreads();
+  } else {
+    __syncwarp();
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+  }
+}
+
+__device__ __forceinline__ void st_remote(uint32_t local_addr, uint32_t rank, double v) {
+  uint32_t ra;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ra) : "r"(local_addr), "r"(rank));
+  asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(ra), "d"(v) : "memory");
+}
+
+// ||tail||_2 of the cone in rows [c0, c1) of a tile from the squares at sq, in
+// ascending order as the reference adds them (eight loaded ahead of their
+// additions).
+__device__ __forceinline__ double cone_norm(uint32_t sq, int c0, int c1) {
+  double ss = 0.0;
+  int r = c0 + 1;
+  for (; r + 8 <= c1; r += 8) {
+    double q[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) q[u] = lds_f64(sq + 8 * (r + u));
+#pragma unroll
+    for (int u = 0; u < 8; ++u) ss = ss + q[u];
+  }
+  for (; r < c1; ++r) ss = ss + lds_f64(sq + 8 * r);
+  return sqrt(ss);
+}
+
+__device__ __forceinline__ uint32_t lds_u16(uint32_t a) {
+  uint16_t v;
+  asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(a) : "memory");
+  return v;
+}
+// the epilogue output that later half-steps gather goes to the CTA's copy
+__device__ __forceinline__ void gather_out(EpiX& e, double* p) { e.x_hat = p; }
+__device__ __forceinline__ void gather_out(EpiQX& e, double* p) { e.w_bar = p; }
+__device__ __forceinline__ void gather_out(EpiQT& e, double* p) { e.tempv = p; }
+__device__ __forceinline__ void gather_out(EpiW2& e, double* p) { e.w = p; }
+__device__ __forceinline__ void gather_out(EpiY& e, double* p) {
+  if (e.ybar_always) e.y_bar = p;  // with Q the w2 half-step gathers y_bar
+  else e.y = p;
+}
+__device__ __forceinline__ void set_full(EpiX& e, int f) { e.full = f; }
+__device__ __forceinline__ void set_full(EpiY& e, int f) { e.full = f; }
+__device__ __forceinline__ void set_full(EpiQX& e, int f) { e.full = f; }
+__device__ __forceinline__ void set_full(EpiQT&, int) {}
+__device__ __forceinline__ void set_full(EpiW2& e, int f) { e.full = f; }
+
+// epilogue inputs through L2: another CTA may have written them
+template <class Epi, int N = Epi::kSlots>
+__device__ __forceinline__ void load_vals_l2(Vals<Epi::kSlots>& o, const Epi& epi, bool cone, int64_t i) {
+#pragma unroll
+  for (int k = 0; k < N; ++k) {
+    const double* p = cone ? epi.cone_src[k] : epi.lin_src[k];
+    o.v[k] = p ? __ldcg(p + i) : 0.0;
+  }
+}
+
+// Copies this CTA's tiles of one side into shared memory.
+__device__ void load_side(const ResSide& s, unsigned char* sm, uint32_t rank, uint32_t C) {
+  const int lane = threadIdx.x & 31;
+  double* val = reinterpret_cast<double*>(sm + s.o_val);
+  uint16_t* col = reinterpret_cast<uint16_t*>(sm + s.o_col);
+  uint64_t* desc = reinterpret_cast<uint64_t*>(sm + s.o_desc);
+  ResTile* tiles = reinterpret_cast<ResTile*>(sm + s.o_tile);
+  ResCones* cones = reinterpret_cast<ResCones*>(sm + s.o_cone);
+  for (int j = threadIdx.x >> 5; (int)rank + (int)C * j < s.nwork; j += kResWarps) {
+    const int t = (int)rank + (int)C * j;
+    const Task tk = s.tasks[t];
+    const TileRun tr = s.runs[t];
+    if (lane == 0) {
+      ResTile x;
+      x.rb = tk.rb;
+      x.nrows = tk.re - tk.rb;
+      x.nnz = tk.nze - tk.nzb;
+      x.soff = tr.soff;
+      x.r0 = tr.r0;
+      x.r1 = tr.r1;
+      x.nonempty = tr.nonempty;
+      x.kind = tk.kind;
+      x.ncones = tk.ncones;
+      x.cone = tk.cone;
+      x.group = tk.group;
+      x.part = tk.part;
+      tiles[j] = x;
+    }
+    desc[32 * j + lane] = s.desc[(int64_t)t * 32 + lane];
+    for (int k = lane; k < tk.ncones; k += 32) {
+      const int c0 = s.cone_start[tk.cone + k] - tk.rb, c1 = s.cone_start[tk.cone + k + 1] - tk.rb;
+      cones[j].start[k] = (uint8_t)c0;
+      if (k == tk.ncones - 1) cones[j].start[k + 1] = (uint8_t)c1;
+      for (int r = c0; r < c1; ++r) cones[j].head[r] = (uint8_t)c0;
+    }
+    // the tile's steps (row mode: of its first and second 32 rows), each
+    // group padded with zeros
+    const int n0 = tr.r0 >= 0 ? tr.r0 : (tk.nze - tk.nzb + 31) >> 5, n1 = tr.r0 >= 0 ? tr.r1 : 0;
+    const int p0 = pad_steps(n0), all = p0 + pad_steps(n1);
+#pragma unroll 4
+    for (int k = 0; k < all; ++k) {
+      const int g = k < p0 ? k : n0 + k - p0;  // step in the plan's arrays
+      const bool in = k < p0 ? k < n0 : k - p0 < n1;
+      val[tr.soff + 32 * k + lane] = in ? __ldcs(s.tval + tr.sbase + 32 * g + lane) : 0.0;
+      col[tr.soff + 32 * k + lane] = in ? (uint16_t)__ldcs(s.tcol + tr.sbase + 32 * g + lane) : (uint16_t)0;
+    }
+  }
+}
+
+// The value rows lane (and lane + 32) wrote to the gathered copy: to the
+// global vector and to the other CTAs' copies.
+__device__ __forceinline__ void publish_rows(double* gout, double* gglob, int rb, int nrows, uint32_t rank,
+                                             uint32_t C) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int h = 0; h < kRowCap / 32; ++h) {
+    const int r = lane + 32 * h;
+    if (r < nrows) {
+      const double v = gout[rb + r];
+      gglob[rb + r] = v;
+      if (C > 1) {
+        const uint32_t a = (uint32_t)__cvta_generic_to_shared(gout + rb + r);
+        for (uint32_t q = 1; q < C; ++q) st_remote(a, (rank + q) & (C - 1), v);
+      }
+    }
+  }
+}
+
+// Sum of one row per lane (row mode): `steps` slots (padded to whole groups of
+// kResUnroll), the lane's own row has `len` of them.  The loads are not
+// conditional (padding is value 0, column 0, its product not used): a branch
+// around each load made every nonzero wait for the one before it.
+__device__ __forceinline__ double row_sum(uint32_t val, uint32_t col, uint32_t xs, int steps, int len) {
+  double sum = 0.0;
+  for (int k0 = 0; k0 < steps; k0 += kResUnroll) {
+    uint32_t c[kResUnroll];
+    double v[kResUnroll], x[kResUnroll];
+#pragma unroll
+    for (int u = 0; u < kResUnroll; ++u) {
+      c[u] = lds_u16(col + 64 * u);
+      v[u] = lds_f64(val + 256 * u);
+    }
+#pragma unroll
+    for (int u = 0; u < kResUnroll; ++u) x[u] = lds_f64(xs + 8 * c[u]);
+#pragma unroll
+    for (int u = 0; u < kResUnroll; ++u) {
+      const double q = v[u] * x[u];
+      sum = sum + (k0 + u < len ? q : 0.0);
+    }
+    col += 64 * kResUnroll;
+    val += 256 * kResUnroll;
+  }
+  return sum;
+}
+
+// Row sums of a tile in runs (process_warp_tile's steps 1 to 3).
+__device__ __forceinline__ void run_sums(uint32_t val, uint32_t col, uint32_t xs, int nnz, uint64_t desc,
+                                         uint64_t nonempty, uint32_t acc, double& acc0, double& acc1) {
+  const int lane = threadIdx.x & 31;
+  const int R = (nnz + 31) >> 5;
+  int my = nnz - lane * R;
+  my = my < 0 ? 0 : (my > R ? R : my);
+  const uint32_t heads = (uint32_t)desc;
+  const int j0 = (int)(desc >> kDescOrdShift);
+  double sum = 0.0;
+  uint32_t next = acc + 8 * j0;                    // slot of the next row to start
+  uint32_t close = acc + 8 * (kRowCap + lane);     // where the segment being summed goes
+  for (int k0 = 0; k0 < R; k0 += kResUnroll) {
+    uint32_t c[kResUnroll];
+    double v[kResUnroll], x[kResUnroll];
+#pragma unroll
+    for (int u = 0; u < kResUnroll; ++u) {
+      c[u] = lds_u16(col + 64 * u);
+      v[u] = lds_f64(val + 256 * u);
+    }
+#pragma unroll
+    for (int u = 0; u < kResUnroll; ++u) x[u] = lds_f64(xs + 8 * c[u]);
+    const uint32_t hb = heads >> k0;
+#pragma unroll
+    for (int u = 0; u < kResUnroll; ++u) {
+      const double q = v[u] * x[u];
+      const bool head = (hb >> u) & 1u;
+      if (head) {
+        sts_f64(close, sum);
+        close = next;
+        next += 8;
+      }
+      sum = (head ? 0.0 : sum) + (k0 + u < my ? q : 0.0);
+    }
+    col += 64 * kResUnroll;
+    val += 256 * kResUnroll;
+  }
+  if (my > 0) sts_f64(close, sum);
+  // rows that span runs: segmented scan of the continuations, then added to
+  // the row's head segment (as the engine)
+  {
+    const bool has_cont = my > 0 && !(heads & 1u);
+    if (__any_sync(0xffffffffu, has_cont)) {
+      const int key = has_cont ? j0 - 1 : -2 - lane;
+      double v = has_cont ? lds_f64(acc + 8 * (kRowCap + lane)) : 0.0;
+#pragma unroll
+      for (int d = 1; d < 32; d <<= 1) {
+        const int ok = __shfl_up_sync(0xffffffffu, key, d);
+        const bool add = lane >= d && ok == key;
+        if (!__any_sync(0xffffffffu, add)) break;
+        const double o = __shfl_up_sync(0xffffffffu, v, d);
+        if (add) v = o + v;
+      }
+      const int nk = __shfl_down_sync(0xffffffffu, key, 1);
+      __syncwarp();
+      if (has_cont && (lane == 31 || nk != key)) sts_f64(acc + 8 * key, lds_f64(acc + 8 * key) + v);
+    }
+    __syncwarp();
+  }
+  {
+    const unsigned lt = (1u << lane) - 1u;
+    const uint64_t ne = nonempty;
+    const unsigned b0 = (unsigned)(ne & 0xffffffffull), b1 = (unsigned)(ne >> 32);
+    if ((b0 >> lane) & 1u) acc0 = lds_f64(acc + 8 * __popc(b0 & lt));
+    if ((b1 >> lane) & 1u) acc1 = lds_f64(acc + 8 * (__popc(b0) + __popc(b1 & lt)));
+    __syncwarp();
+  }
+}
+
+// One tile with nonzeros: row sums, then the epilogue (whole rows and cones)
+// or the raw values and norm share (a slice of a split cone).
+template <class E>
+__device__ __forceinline__ void res_tile(const ResSide& s, unsigned char* sm, E& epi, int j, uint32_t xs,
+                                         ResWs& ws, double* gout, double* gglob, uint32_t rank, uint32_t C) {
+  const int lane = threadIdx.x & 31;
+  const ResTile* tp = reinterpret_cast<const ResTile*>(sm + s.o_tile) + j;
+  const int rb = tp->rb, nrows = tp->nrows;
+  const uint64_t desc = reinterpret_cast<const uint64_t*>(sm + s.o_desc)[32 * j + lane];
+  const bool part = tp->kind == TASK_CONE_PART;
+  const bool cone = E::kCones && (part || tp->cone >= 0);
+  Vals<E::kSlots> v0, v1;
+  if (lane < nrows) load_vals_l2<E>(v0, epi, cone, rb + lane);
+  if (lane + 32 < nrows) load_vals_l2<E>(v1, epi, cone, rb + lane + 32);
+  const uint32_t smb = (uint32_t)__cvta_generic_to_shared(sm);
+  const uint32_t val = smb + s.o_val + 8 * (tp->soff + lane), col = smb + s.o_col + 2 * (tp->soff + lane);
+  double acc0 = 0.0, acc1 = 0.0;  // sums of rows rb + lane and rb + lane + 32
+  const int r0 = tp->r0;
+  if (r0 >= 0) {
+    // row mode: the lane's rows, in column order
+    acc0 = row_sum(val, col, xs, r0, (int)(desc & 0xffff));
+    const int r1 = tp->r1;
+    const int o1 = 32 * pad_steps(r0);
+    if (r1 > 0) acc1 = row_sum(val + 8 * o1, col + 2 * o1, xs, r1, (int)((desc >> 16) & 0xffff));
+  } else {
+    run_sums(val, col, xs, tp->nnz, desc, tp->nonempty, (uint32_t)__cvta_generic_to_shared(ws.acc), acc0, acc1);
+  }
+  Red red;
+  if (!cone) {
+    if (lane < nrows) epi.linear(rb + lane, acc0, v0, red);
+    if (lane + 32 < nrows) epi.linear(rb + lane + 32, acc1, v1, red);
+  } else if (part) {
+    // raw values and this slice's share of ||tail||^2 (big_norm_share)
+    const int head = s.big[tp->group].rb;
+    double sq = 0.0;
+    if (lane < nrows) {
+      const double r = epi.cone_raw(rb + lane, acc0, v0, red);
+      s.raw[rb + lane] = r;
+      if (rb + lane != head) sq = r * r;
+    }
+    if (lane + 32 < nrows) {
+      const double r = epi.cone_raw(rb + lane + 32, acc1, v1, red);
+      s.raw[rb + lane + 32] = r;
+      if (rb + lane + 32 != head) sq = sq + r * r;
+    }
+    const double tot = warp_sum_bcast(sq);
+    if (lane == 0) s.cpart[s.big[tp->group].part_base + tp->part] = tot;
+    return;
+  } else {
+    const ResCones& cn = reinterpret_cast<const ResCones*>(sm + s.o_cone)[j];
+    const uint32_t raw = smem_addr(ws.acc), sqa = smem_addr(ws.sq);
+    double w0 = 0.0, w1 = 0.0;
+    if (lane < nrows) {
+      w0 = epi.cone_raw(rb + lane, acc0, v0, red);
+      sts_f64(raw + 8 * lane, w0);
+      sts_f64(sqa + 8 * lane, w0 * w0);
+    }
+    if (lane + 32 < nrows) {
+      w1 = epi.cone_raw(rb + lane + 32, acc1, v1, red);
+      sts_f64(raw + 8 * (lane + 32), w1);
+      sts_f64(sqa + 8 * (lane + 32), w1 * w1);
+    }
+    __syncwarp();
+    // one lane per cone
+    for (int k = lane; k < tp->ncones; k += 32) {
+      const int c0 = cn.start[k], c1 = cn.start[k + 1];
+      sts_f64(sqa + 8 * c0, cone_norm(sqa, c0, c1));
+    }
+    __syncwarp();
+    if (lane < nrows) {
+      const int h = cn.head[lane];
+      epi.cone_apply(rb + lane, w0, lds_f64(raw + 8 * h), lds_f64(sqa + 8 * h), lane == h, v0, red);
+    }
+    if (lane + 32 < nrows) {
+      const int r = lane + 32, h = cn.head[r];
+      epi.cone_apply(rb + r, w1, lds_f64(raw + 8 * h), lds_f64(sqa + 8 * h), r == h, v1, red);
+    }
+    __syncwarp();
+  }
+  publish_rows(gout, gglob, rb, nrows, rank, C);
+}
+
+// Projection of 64 rows of a split cone, after the barrier that follows its
+// slices: every apply tile adds the shares itself, in publish_big_norm's
+// order.
+template <class E>
+__device__ __forceinline__ void res_apply(const ResSide& s, E& epi, int t, double* gout, double* gglob, uint32_t rank,
+                                          uint32_t C) {
+  const int lane = threadIdx.x & 31;
+  const Task tk = s.tasks[t];
+  const BigCone bc = s.big[tk.group];
+  const int nrows = tk.re - tk.rb;
+  Vals<E::kSlots> v0, v1;
+  double rv0 = 0.0, rv1 = 0.0;
+  constexpr int kN = ApplySlots<E>::value;
+  if (lane < nrows) {
+    load_vals_l2<E, kN>(v0, epi, true, tk.rb + lane);
+    rv0 = __ldcg(s.raw + tk.rb + lane);
+  }
+  if (lane + 32 < nrows) {
+    load_vals_l2<E, kN>(v1, epi, true, tk.rb + lane + 32);
+    rv1 = __ldcg(s.raw + tk.rb + lane + 32);
+  }
+  double part = 0.0;
+  for (int q = lane; q < bc.nparts; q += 32) part = part + __ldcg(s.cpart + bc.part_base + q);
+  const double tv = __ldcg(s.raw + bc.rb);
+  const double ns = sqrt(warp_sum_bcast(part));
+  Red red;
+  if (lane < nrows) epi.cone_apply(tk.rb + lane, rv0, tv, ns, tk.rb + lane == bc.rb, v0, red);
+  if (lane + 32 < nrows) epi.cone_apply(tk.rb + lane + 32, rv1, tv, ns, tk.rb + lane + 32 == bc.rb, v1, red);
+  publish_rows(gout, gglob, tk.rb, nrows, rank, C);
+}
+
+template <class E>
+__device__ __forceinline__ void res_stage(const RStage<E>& st, const ResArgs& a, unsigned char* sm,
+                                          const DevState* cur, bool last, ResWs& ws, uint32_t rank, uint32_t C) {
+  if (!st.on) return;
+  const ResSide& s = a.side[st.side];
+  E e = st.e;
+  double* gout = reinterpret_cast<double*>(sm + st.gout);
+  const uint32_t xs = (uint32_t)__cvta_generic_to_shared(sm + st.gin);
+  set_full(e, last ? 1 : 0);
+  gather_out(e, gout);
+  e.setup(cur);
+  for (int j = threadIdx.x >> 5; (int)rank + (int)C * j < s.nwork; j += kResWarps)
+    res_tile<E>(s, sm, e, j, xs, ws, gout, st.gglob, rank, C);
+  if constexpr (E::kCones) {
+    if (s.nbig > 0) {
+      res_sync(C);
+      for (int j = threadIdx.x >> 5; s.nwork + (int)rank + (int)C * j < s.ntasks; j += kResWarps)
+        res_apply<E>(s, e, s.nwork + (int)rank + (int)C * j, gout, st.gglob, rank, C);
+    }
+  }
+  res_sync(C);
+}
+
+template <class E0, class E1, class E2, class E3>
+__global__ void __launch_bounds__(kResThreads, 1)
+    resident_kernel(const __grid_constant__ ResArgs a, const __grid_constant__ RStage<E0> s0,
+                    const __grid_constant__ RStage<E1> s1, const __grid_constant__ RStage<E2> s2,
+                    const __grid_constant__ RStage<E3> s3) {
+  extern __shared__ __align__(16) unsigned char sm[];
+  const uint32_t rank = cluster_rank(), C = cluster_size();
+  ResWs& ws = reinterpret_cast<ResWs*>(sm + a.o_ws)[threadIdx.x >> 5];
+  DevState* st = reinterpret_cast<DevState*>(sm + a.o_state);
+  for (int i = 0; i < a.nsides; ++i) load_side(a.side[i], sm, rank, C);
+  {
+    double* g = reinterpret_cast<double*>(sm + a.g0_off);
+    for (int i = threadIdx.x; i < a.g0_len; i += kResThreads) g[i] = a.g0[i];
+  }
+  if (threadIdx.x == 0) st[0] = st[1] = *a.st;
+  res_sync(C);
+  const long long inner = st[0].inner;
+  for (int it = 0; it < a.iters; ++it) {
+    const bool last = a.full_last && it + 1 == a.iters;
+    // the next iteration's scalars, in the copy that no warp reads now
+    if (threadIdx.x == 0) st[(it + 1) & 1].inner = inner + it + 1;
+    const DevState* cur = st + (it & 1);
+    res_stage(s0, a, sm, cur, last, ws, rank, C);
+    res_stage(s1, a, sm, cur, last, ws, rank, C);
+    res_stage(s2, a, sm, cur, last, ws, rank, C);
+    res_stage(s3, a, sm, cur, last, ws, rank, C);
+  }
+  if (rank == 0 && threadIdx.x == 0) a.st->inner = inner + a.iters;
+}
+
+// ---------------------------------------------------------------------------
+// Host side
+// ---------------------------------------------------------------------------
+int align16(int64_t b) { return (int)((b + 15) & ~(int64_t)15); }
+
+// Shared-memory bytes of a batch on C CTAs, with the largest CTA's slots and
+// tiles per side, and the offsets (when given).
+int64_t resident_layout(const Ctx* c, const ResidentShape& r, ResArgs* a, int* goff) {
+  int64_t o = 0;
+  auto take = [&](int64_t bytes) {
+    const int64_t at = o;
+    o = align16(o + bytes);
+    return (int)at;
+  };
+  const int o_state = take(2 * sizeof(DevState)), o_ws = take(kResWarps * sizeof(ResWs));
+  if (a) {
+    a->o_state = o_state;
+    a->o_ws = o_ws;
+  }
+  // gathered vectors: y, x_hat; with Q y_bar, w (tempv in the same place: w is
+  // gathered by the first half-step only), w_bar
+  const int64_t len[3] = {c->m, c->n, c->n};
+  for (int k = 0; k < (c->has_q ? 3 : 2); ++k) {
+    const int at = take(8 * std::max<int64_t>(len[k], 1));
+    if (goff) goff[k] = at;
+  }
+  for (int i = 0; i < (c->has_q ? 3 : 2); ++i) {
+    const int ov = take(8LL * r.slots[i]), od = take(256LL * r.tiles[i]);
+    const int ot = take((int64_t)sizeof(ResTile) * r.tiles[i]), oc = take((int64_t)sizeof(ResCones) * r.tiles[i]);
+    const int ocol = take(2LL * r.slots[i]);
+    if (a) {
+      a->side[i].o_val = ov;
+      a->side[i].o_desc = od;
+      a->side[i].o_tile = ot;
+      a->side[i].o_cone = oc;
+      a->side[i].o_col = ocol;
+    }
+  }
+  return o;
+}
+
+int nwork_of(const Plan& p) {
+  int n = (int)p.tasks.size();
+  while (n > 0 && p.tasks[n - 1].kind == TASK_CONE_APPLY) --n;
+  return n;
+}
+
+using NoQKernel = decltype(&resident_kernel<EpiX, EpiY, EpiY, EpiY>);
+using QKernel = decltype(&resident_kernel<EpiQX, EpiQT, EpiY, EpiW2>);
+
+cudaLaunchConfig_t resident_config(int C, int64_t smem, cudaStream_t stream, cudaLaunchAttribute* attr) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)C);
+  cfg.blockDim = dim3(kResThreads);
+  cfg.dynamicSmemBytes = (size_t)smem;
+  cfg.stream = stream;
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = (unsigned)C;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cfg;
+}
+
+// The kernel's attributes are set once per device; true if a cluster of C
+// CTAs with the full shared memory can run on it.
+template <class K>
+bool cluster_fits(int device, K kernel, int C) {
+  static std::mutex mu;
+  static std::set<int> ready;                    // devices whose attributes are set
+  static std::set<std::pair<int, int>> yes, no;  // (device, CTAs)
+  std::lock_guard<std::mutex> lk(mu);
+  if (yes.count({device, C})) return true;
+  if (no.count({device, C})) return false;
+  if (!ready.count(device)) {
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kResSmemMax) != cudaSuccess ||
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
+      (void)cudaGetLastError();
+      return false;
+    }
+    ready.insert(device);
+  }
+  cudaLaunchAttribute attr[1];
+  const cudaLaunchConfig_t cfg = resident_config(C, kResSmemMax, nullptr, attr);
+  int n = 0;
+  const bool ok = cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) == cudaSuccess && n > 0;
+  if (!ok) (void)cudaGetLastError();
+  (ok ? yes : no).insert({device, C});
+  return ok;
+}
+
+}  // namespace
+
+// The cluster size for a problem of these sizes and the soft tile caps that
+// spread its rows over the cluster's warps (0 CTAs: does not fit).  The
+// smallest cluster that holds the problem: a larger one spreads the same
+// chains over more barriers (measured on B200, us per iteration on 1 / 2 / 4 /
+// 8 / 16 CTAs: n = 61 4.3 / 5.3 / 5.1 / 5.2 / 5.1, n = 400 9.9 / 10.5 / 10.2 /
+// 10.3 / 10.9), and the other SMs serve other contexts.
+ResidentShape resident_estimate(int64_t m, int64_t n, int64_t nnz, int64_t qnnz, bool has_q) {
+  ResidentShape r;
+  if (n > 65536 || m > 65536 || n == 0) return r;
+  const int64_t gather = 8 * (m + n + (has_q ? n : 0));
+  for (int C = 1; C <= kResMaxCtas; C *= 2) {
+    const int64_t warps = (int64_t)C * kResWarps;
+    const int64_t cap = std::min<int64_t>((nnz * 5 / 4 / warps + 127) / 128 * 128, kNnzTile);
+    const int64_t tiles = 3 * kResWarps;  // about one per warp and side (resident_plan has the exact sizes)
+    const int64_t bytes = gather + (2 * nnz + qnnz) / C * 11 + tiles * 440 + kResWarps * (int64_t)sizeof(ResWs) + 2048;
+    if (bytes > kResSmemMax) continue;
+    r.ctas = C;
+    r.soft_nnz = (int)std::max<int64_t>(cap, 128);
+    r.soft_rows = 32;  // one row per lane
+    return r;
+  }
+  return r;
+}
+
+// Slot offsets of the plans' tiles in their CTA's shared memory (TileRun.pad)
+// for the cluster size of c->res, raised until the batch fits; c->res.ctas
+// becomes 0 when it does not (or a side has a row longer than a tile).
+void resident_plan(Ctx* c) {
+  ResidentShape& r = c->res;
+  Plan* plans[3] = {&c->planX, &c->planY, &c->planQ};
+  const int ns = c->has_q ? 3 : 2;
+  for (int i = 0; i < ns; ++i)
+    if (!plans[i]->lng.empty()) r.ctas = 0;
+  for (; r.ctas > 0; r.ctas = r.ctas < kResMaxCtas ? 2 * r.ctas : 0) {
+    const int C = r.ctas;
+    for (int i = 0; i < ns; ++i) {
+      Plan& p = *plans[i];
+      int64_t used[kResMaxCtas] = {0};
+      const int nw = nwork_of(p);
+      for (int t = 0; t < nw; ++t) {
+        TileRun& tr = p.runs[t];
+        tr.soff = (int32_t)used[t % C];
+        used[t % C] += 32 * (int64_t)(tr.r0 >= 0 ? pad_steps(tr.r0) + pad_steps(tr.r1)
+                                                 : pad_steps((p.tasks[t].nze - p.tasks[t].nzb + 31) / 32));
+      }
+      r.slots[i] = (int)*std::max_element(used, used + C);
+      r.tiles[i] = (nw + C - 1) / C;
+    }
+    if (resident_layout(c, r, nullptr, nullptr) <= kResSmemMax) return;
+  }
+}
+
+bool resident_eligible(const Ctx* c) {
+  if (c->res.ctas == 0 || c->precision != HPR_PREC_FP64) return false;
+  if (c->q_kind != HPR_Q_NONE && c->q_kind != HPR_Q_CSR) return false;
+  return c->has_q ? cluster_fits<QKernel>(c->device, resident_kernel<EpiQX, EpiQT, EpiY, EpiW2>, c->res.ctas)
+                  : cluster_fits<NoQKernel>(c->device, resident_kernel<EpiX, EpiY, EpiY, EpiY>, c->res.ctas);
+}
+
+// k iterations (the last one full when full_last) in one launch.
+int launch_resident(Ctx* c, int64_t k, bool full_last) {
+  HPR_TRY(prepare_engine(c));
+  IterEpis E;
+  make_iter_epis(c, false, E);
+  ResArgs a = ResArgs();
+  int g[3] = {0, 0, 0};
+  const int64_t smem = resident_layout(c, c->res, &a, g);
+  const Plan* plans[3] = {&c->planX, &c->planY, &c->planQ};
+  const int32_t* cs[3] = {c->d_var_start, c->d_con_start, c->d_var_start};
+  a.nsides = c->has_q ? 3 : 2;
+  for (int i = 0; i < a.nsides; ++i) {
+    const PlanView v = view_of(*plans[i], cs[i]);
+    ResSide& s = a.side[i];
+    s.tasks = v.tasks;
+    s.runs = v.runs;
+    s.desc = v.desc;
+    s.tcol = v.tcol;
+    s.tval = v.tval;
+    s.cone_start = v.cone_start;
+    s.big = v.big;
+    s.raw = v.raw;
+    s.cpart = v.cpart;
+    s.ntasks = v.ntasks;
+    s.nwork = nwork_of(*plans[i]);
+    s.nbig = v.nbig;
+  }
+  a.st = c->d_state;
+  a.g0 = c->has_q ? c->w : c->y;
+  a.g0_off = c->has_q ? g[1] : g[0];
+  a.g0_len = (int)(c->has_q ? c->n : c->m);
+  const int hy = c->m > 0 ? 1 : 0;
+  cudaLaunchAttribute attr[1];
+  const cudaLaunchConfig_t cfg = resident_config(c->res.ctas, smem, c->stream, attr);
+  for (int64_t done = 0; done < k;) {
+    a.iters = (int)std::min<int64_t>(k - done, 1 << 20);
+    a.full_last = (full_last && done + a.iters == k) ? 1 : 0;
+    if (!c->has_q) {
+      const RStage<EpiX> sx{E.ex, 0, g[0], g[1], c->x_hat, 1};
+      const RStage<EpiY> sy{E.ey, 1, g[1], g[0], c->y, hy};
+      const RStage<EpiY> off{E.ey, 1, g[1], g[0], c->y, 0};
+      HPR_CUDA(c, cudaLaunchKernelEx(&cfg, resident_kernel<EpiX, EpiY, EpiY, EpiY>, a, sx, sy, off, off));
+    } else {
+      const RStage<EpiQX> sq{E.eq, 2, g[1], g[2], c->w_bar, 1};
+      const RStage<EpiQT> st{E.et, 2, g[2], g[1], c->tempv, hy};
+      const RStage<EpiY> sy{E.ey, 1, g[1], g[0], c->y_bar, hy};
+      const RStage<EpiW2> sw{E.e2, 0, g[0], g[1], c->w, 1};
+      HPR_CUDA(c, cudaLaunchKernelEx(&cfg, resident_kernel<EpiQX, EpiQT, EpiY, EpiW2>, a, sq, st, sy, sw));
+    }
+    c->launches++;
+    done += a.iters;
+  }
+  return HPR_OK;
+}
+
+}  // namespace hpr

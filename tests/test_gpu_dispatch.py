@@ -37,3 +37,36 @@ def _check(model, iters=10, tol=1e-12, schedule="engine"):
 def test_one_wave_of_wide_tiles_and_more(scale):
     """About 1,600 to 2,700 tiles per side: the two-CTA form up to 2,368."""
     _check(instances.config1(3, scale=scale))
+
+
+# (rows of A about n / 2, 3.5% dense: one CTA, then clusters of 2 to 16 CTAs,
+# then past the largest; 48 to 56 and 1,100 have cones split over tiles or one
+# tile's 33rd row)
+@pytest.mark.parametrize("n", [50, 56, 120, 400, 690, 803, 1100, 1700, 2300, 2900, 3600])
+@pytest.mark.parametrize("diag_q", [False, True])
+def test_cluster_resident_batches(n, diag_q):
+    _check(instances.small_socp(100 + n, n=n, diag_q=diag_q), iters=40, tol=1e-11, schedule="auto")
+
+
+@pytest.mark.parametrize("n", [40, 400, 1200, 3000])
+def test_cluster_resident_batches_general_q(n):
+    _check(instances.qp_csr(n, n=n, density=0.02 if n < 2000 else 0.01), iters=40, tol=1e-11, schedule="auto")
+
+
+@pytest.mark.parametrize("n", [60, 400, 1500])
+def test_resident_and_engine_agree_to_the_bit(n):
+    from hprsocp_b200 import Context
+    model = instances.small_socp(7 + n, n=n, diag_q=False)
+    res = []
+    for mode in ("engine", "auto"):
+        with Context(model) as g:
+            g.set_schedule(mode)
+            info = g.scale(HPRSOCP_parameters(verbose=False))
+            g.set_sigma_lambda(info["norm_b"] / info["norm_c"], 1.05 * g.power_A(), 0.0)
+            g.set_inner(0)
+            g.iterate(70, True)
+            g.iterate(1, False)
+            g.iterate(30, True)
+            res.append([g.get(v) for v in VECS] + [np.array(g.scalars())])
+    for a, b in zip(*res):
+        assert np.array_equal(a, b)
