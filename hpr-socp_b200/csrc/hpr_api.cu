@@ -471,6 +471,7 @@ int solve_host_loop(Ctx* c, const hpr_params* P, const SolveSetup& S, hpr_result
   const int64_t ci = P->check_iter;
   int status = -1;
   int64_t iter = 0;
+  bool have_lanes = false;  // the last batch computed the residual lanes of its last iterate
   // Reduced-precision stream: residuals, restart and sigma logic stay FP64;
   // the SpMV stream itself switches to FP64 for the finish once the KKT
   // measure is within `switch_factor` of the tolerance or has stopped
@@ -485,7 +486,12 @@ int solve_host_loop(Ctx* c, const hpr_params* P, const SolveSetup& S, hpr_result
     // ---- the event iteration `iter` (residual check or print)
     double el = now_s() - t0;
     bool print_yes = is_print_iter(iter, P) || el > P->time_limit;
-    if (iter % ci == 0 || print_yes) HPR_TRY(launch_residuals(c, iter == 0, &rs));
+    if (iter % ci == 0 || print_yes) {
+      // the batch that led here may have left the residual lanes
+      if (have_lanes) HPR_TRY(finish_residuals(c, false, kCheckLanes, &rs));
+      else HPR_TRY(launch_residuals(c, iter == 0, &rs));
+    }
+    have_lanes = false;
     if (rs.KKTx_and_gap_org_bar != rs.KKTx_and_gap_org_bar)
       return set_err(c, HPR_E_NUMERIC, "NaN in the KKT residuals at iteration " + std::to_string(iter));
     if (ckpt && (iter % ci == 0 || print_yes)) HPR_TRY(ckpt_track(ckpt.get(), iter, c->sigma, rs));
@@ -540,7 +546,7 @@ int solve_host_loop(Ctx* c, const hpr_params* P, const SolveSetup& S, hpr_result
     while (!(next % ci == 0 || is_print_iter(next, P))) ++next;
     if (R.flag > 0) {
       // the restart iteration's own step is full and needs the M-norm
-      HPR_TRY(run_iterations(c, 1, true));
+      HPR_TRY(run_iterations(c, 1, true, iter + 1 == next, &have_lanes));
       double mn;
       HPR_TRY(launch_mnorm(c, &mn));
       R.last_gap = std::min(mn, R.last_gap);
@@ -548,12 +554,12 @@ int solve_host_loop(Ctx* c, const hpr_params* P, const SolveSetup& S, hpr_result
       R.inner += 1;
       iter += 1;
       if (iter < next) {
-        HPR_TRY(run_iterations(c, next - iter, true));
+        HPR_TRY(run_iterations(c, next - iter, true, true, &have_lanes));
         R.inner += next - iter;
         if (next % ci == 0) HPR_TRY(launch_mnorm(c, &R.current_gap));
       }
     } else {
-      HPR_TRY(run_iterations(c, next - iter, true));
+      HPR_TRY(run_iterations(c, next - iter, true, true, &have_lanes));
       R.inner += next - iter;
       if (next % ci == 0) HPR_TRY(launch_mnorm(c, &R.current_gap));
     }
@@ -997,6 +1003,8 @@ int hpr_upload(hpr_ctx* h, const hpr_problem* p) {
   HPR_TRY(zero_vec(c, &c->d_red_out, 64));
   HPR_TRY(dev_alloc_n(c, &c->d_red2, (int64_t)kWideReduceCtas * kMaxRed));
   int64_t need = (int64_t)kRedGrid * kMaxRed;
+  // a cluster-resident batch's check keeps both sides' slots
+  if (c->res.ctas > 0) need = std::max(need, (int64_t)(c->planX.nslots() + c->planY.nslots()) * kMaxRed);
   if (need > c->red_slots) {
     dev_free(c, c->d_red);
     c->d_red = nullptr;

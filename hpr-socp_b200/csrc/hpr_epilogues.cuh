@@ -560,6 +560,26 @@ inline void make_iter_epis(Ctx* c, bool full, IterEpis& E) {
 }
 
 
+// Epilogues of the residual passes (compute_residuals!, algorithm.jl:113-196).
+struct ResidualEpis {
+  EpiRd rd{};
+  EpiRp rp{};
+};
+
+inline void make_residual_epis(Ctx* c, ResidualEpis& R) {
+  const double* dsrc[5] = {c->c, c->z_bar, c->x_bar, c->col_norm, c->has_q ? c->Qx : nullptr};
+  for (int k = 0; k < 5; ++k) R.rd.lin_src[k] = R.rd.cone_src[k] = dsrc[k];
+  R.rd.hasq = c->has_q ? 1 : 0;
+  R.rd.cs = c->c_scale;
+  const double* psrc[5] = {c->AL, c->AU, c->row_norm, c->y_bar, c->s};
+  const double* pcone[5] = {c->soc_rhs_full, nullptr, c->row_norm, c->y_bar, c->s};
+  for (int k = 0; k < 5; ++k) {
+    R.rp.lin_src[k] = psrc[k];
+    R.rp.cone_src[k] = pcone[k];
+  }
+  R.rp.bs = c->b_scale;
+}
+
 // ---------------------------------------------------------------------------
 // Stages of the single-CTA kernels: one matrix side, its plan and the
 // partial / full epilogues of one half-step.  A problem whose sides have at

@@ -334,7 +334,9 @@ int ensure_tiled(Ctx* c, const DevCSR& M, const Plan& p, bool build = true);
 int prepare_engine(Ctx* c, bool build = true);
 PlanView view_of(const Plan& p, const int32_t* cone_start);
 int launch_iteration(Ctx* c, bool full);
-int run_iterations(Ctx* c, int64_t k, bool full_last);
+// check: the caller wants the residuals of the last iterate next; *checked is
+// true when their lanes were computed with the batch (finish_residuals)
+int run_iterations(Ctx* c, int64_t k, bool full_last, bool check = false, bool* checked = nullptr);
 // true when run_iterations may use the single-CTA multi-iteration kernel
 // (then no partial-iteration graph is captured)
 bool uses_fused_iterations(const Ctx* c);
@@ -342,14 +344,20 @@ bool uses_fused_iterations(const Ctx* c);
 ResidentShape resident_estimate(int64_t m, int64_t n, int64_t nnz, int64_t qnnz, bool has_q);
 void resident_plan(Ctx* c);  // after the plans are built, before upload_plan
 bool resident_eligible(const Ctx* c);
-int launch_resident(Ctx* c, int64_t k, bool full_last);
+int launch_resident(Ctx* c, int64_t k, bool full_last, bool check);
 int launch_residuals(Ctx* c, bool include_bounds, hpr_residuals* out);
+// reads the residual lanes back (Rd's from lane `base` of d_red_out, Rp's from
+// base + 8) and forms the residuals
+int finish_residuals(Ctx* c, bool include_bounds, int base, hpr_residuals* out);
+constexpr int kCheckLanes = 44;  // where a cluster-resident batch leaves them
 int launch_residuals_noalloc(Ctx* c, bool include_bounds, hpr_residuals* out);
 int launch_mnorm(Ctx* c, double* out);
 int launch_sigma_terms(Ctx* c, double* a, double* b, double* cc, double* d);
 int launch_golden_diag(Ctx* c, double a, double b, double lo, double hi,
                        double tol, double* out);
 int launch_restart(Ctx* c);
+// the power iteration of a cluster-resident problem; *done = false: does not fit
+int launch_resident_power(Ctx* c, int maxit, double tol, double* lam, bool* done);
 int launch_power_A(Ctx* c, int maxit, double tol, double* lam);
 int launch_power_Q(Ctx* c, int maxit, double tol, double* lam);
 int push_state(Ctx* c);

@@ -653,13 +653,15 @@ bool uses_fused_iterations(const Ctx* c) {
   return mode != HPR_SCHEDULE_ENGINE;
 }
 
-int run_iterations(Ctx* c, int64_t k, bool full_last) {
+int run_iterations(Ctx* c, int64_t k, bool full_last, bool check, bool* checked) {
+  if (checked) *checked = false;
   if (k <= 0) return HPR_OK;
   int64_t l0 = c->launches;
   HPR_CUDA(c, cudaEventRecord(c->ev0, c->stream));
   int mode = HPR_SCHEDULE_ENGINE;
   if (c->schedule != HPR_SCHEDULE_ENGINE && resident_eligible(c)) {
-    HPR_TRY(launch_resident(c, k, full_last));
+    HPR_TRY(launch_resident(c, k, full_last, check && full_last));
+    if (checked) *checked = check && full_last;
     HPR_CUDA(c, cudaEventRecord(c->ev1, c->stream));
     c->inner += k;
     c->last_launches = c->launches - l0;
@@ -724,27 +726,14 @@ __global__ void bounds_cone_kernel(int64_t ncones, const int32_t* vs, const doub
 }  // namespace
 
 int launch_residuals(Ctx* c, bool include_bounds, hpr_residuals* r) {
-  const double bs = c->b_scale, cs = c->c_scale;
+  const double bs = c->b_scale;
   const bool skipq = !c->has_q;
   // offsets in d_red_out: [0..5] Rd lanes, [8..12] Rp lanes, [16] bounds
   if (!skipq) HPR_TRY(qmap(c, c->x_bar, c->Qx, c->ftmp));
-  EpiRd ed{};
-  const double* dsrc[5] = {c->c, c->z_bar, c->x_bar, c->col_norm, skipq ? nullptr : c->Qx};
-  for (int k = 0; k < 5; ++k) ed.lin_src[k] = ed.cone_src[k] = dsrc[k];
-  ed.hasq = skipq ? 0 : 1;
-  ed.cs = cs;
-  HPR_TRY(engine_launch(c, c->AT, c->planX, c->d_var_start, c->y_bar, nullptr, ed, false, true, 0));
-  if (c->m > 0) {
-    EpiRp ep{};
-    const double* psrc[5] = {c->AL, c->AU, c->row_norm, c->y_bar, c->s};
-    const double* pcone[5] = {c->soc_rhs_full, nullptr, c->row_norm, c->y_bar, c->s};
-    for (int k = 0; k < 5; ++k) {
-      ep.lin_src[k] = psrc[k];
-      ep.cone_src[k] = pcone[k];
-    }
-    ep.bs = bs;
-    HPR_TRY(engine_launch(c, c->A, c->planY, c->d_con_start, c->x_bar, nullptr, ep, false, true, 8));
-  }
+  ResidualEpis R;
+  make_residual_epis(c, R);
+  HPR_TRY(engine_launch(c, c->AT, c->planX, c->d_var_start, c->y_bar, nullptr, R.rd, false, true, 0));
+  if (c->m > 0) HPR_TRY(engine_launch(c, c->A, c->planY, c->d_con_start, c->x_bar, nullptr, R.rp, false, true, 8));
   if (include_bounds) {
     bounds_box_kernel<<<592, kThreads, 0, c->stream>>>(c->n, c->l, c->u, c->x_bar, c->col_norm, bs, c->dx);
     int64_t nv = (int64_t)c->h_var_idx.size() - 1;
@@ -754,8 +743,14 @@ int launch_residuals(Ctx* c, bool include_bounds, hpr_residuals* r) {
     HPR_CUDA(c, cudaGetLastError());
     HPR_TRY(vec_reduce<1, 1>(c, c->n, AbsMaxF{c->dx}, 16));
   }
-  HPR_TRY(fetch_red(c, 17));
-  const double* h = c->h_red_out;
+  return finish_residuals(c, include_bounds, 0, r);
+}
+
+int finish_residuals(Ctx* c, bool include_bounds, int base, hpr_residuals* r) {
+  const double bs = c->b_scale, cs = c->c_scale;
+  const bool skipq = !c->has_q;
+  HPR_TRY(fetch_red(c, base + 17));
+  const double* h = c->h_red_out + base;
   auto jmax = [](double a, double b) { return (a != a) ? a : ((b != b) ? b : (a > b ? a : b)); };
   double qx_dot = skipq ? 0.0 : h[5];
   r->primal_obj_bar = bs * cs * (h[3] + 0.5 * qx_dot) + c->obj_constant;
@@ -1242,6 +1237,9 @@ int launch_power_A(Ctx* c, int maxit, double tol, double* lam) {
     *lam = 0.0;
     return HPR_OK;
   }
+  bool done = false;
+  HPR_TRY(launch_resident_power(c, maxit, tol, lam, &done));
+  if (done) return HPR_OK;
   if (one_cta_plan(c->planX) && one_cta_plan(c->planY) && kEngineSmem <= kSmemOptinMax) return power_fused_A(c, maxit, tol, lam);
   return power_two_pass_A(c, maxit, tol, lam);
 }

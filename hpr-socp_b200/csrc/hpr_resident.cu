@@ -23,6 +23,7 @@
 #include <algorithm>
 #include <mutex>
 #include <set>
+#include <vector>
 
 #include "hpr_epilogues.cuh"
 
@@ -33,7 +34,7 @@ namespace {
 constexpr int kResWarps = 16;
 constexpr int kResThreads = kResWarps * 32;
 constexpr int kResMaxCtas = 16;
-constexpr int kResSmemMax = 226 * 1024;
+constexpr int kResSmemMax = 226 * 1024;  // with the static reduction arrays within 227 KB
 constexpr int kResUnroll = 4;  // nonzeros per lane per step
 
 __host__ __device__ inline int pad_steps(int n) { return (n + kResUnroll - 1) / kResUnroll * kResUnroll; }
@@ -76,6 +77,19 @@ struct RStage {
   int side, gin, gout;
   double* gglob;
   int on;
+  double* slots;  // reduction slots of the side's tiles (epilogues with reductions)
+};
+
+// The residual check after a batch (compute_residuals!): the half-steps of
+// launch_residuals and where their lanes go.
+struct ResCheck {
+  RStage<EpiPlain> qx;
+  RStage<EpiRd> rd;
+  RStage<EpiRp> rp;
+  const double *x_bar, *y_bar;
+  int n, m, on;
+  int slots_x, slots_y;
+  double* out;  // Rd lanes at 0, Rp lanes at 8
 };
 
 struct ResArgs {
@@ -153,6 +167,12 @@ __device__ __forceinline__ void gather_out(EpiY& e, double* p) {
   if (e.ybar_always) e.y_bar = p;  // with Q the w2 half-step gathers y_bar
   else e.y = p;
 }
+__device__ __forceinline__ void gather_out(EpiPlain& e, double* p) { e.out = p; }
+__device__ __forceinline__ void gather_out(EpiRd&, double*) {}
+__device__ __forceinline__ void gather_out(EpiRp&, double*) {}
+__device__ __forceinline__ void set_full(EpiPlain&, int) {}
+__device__ __forceinline__ void set_full(EpiRd&, int) {}
+__device__ __forceinline__ void set_full(EpiRp&, int) {}
 __device__ __forceinline__ void set_full(EpiX& e, int f) { e.full = f; }
 __device__ __forceinline__ void set_full(EpiY& e, int f) { e.full = f; }
 __device__ __forceinline__ void set_full(EpiQX& e, int f) { e.full = f; }
@@ -166,6 +186,16 @@ __device__ __forceinline__ void load_vals_l2(Vals<Epi::kSlots>& o, const Epi& ep
   for (int k = 0; k < N; ++k) {
     const double* p = cone ? epi.cone_src[k] : epi.lin_src[k];
     o.v[k] = p ? __ldcg(p + i) : 0.0;
+  }
+}
+
+// The reduction lanes of a tile to its slot.
+template <class E>
+__device__ __forceinline__ void put_red(double* slots, int slot, Red& red) {
+  if constexpr (E::kNRed > 0) {
+    warp_reduce<E::kNRed, E::kMaxMask>(red);
+    if ((threadIdx.x & 31) == 0)
+      for (int k = 0; k < E::kNRed; ++k) slots[(int64_t)slot * kMaxRed + k] = red.v[k];
   }
 }
 
@@ -337,7 +367,7 @@ __device__ __forceinline__ void run_sums(uint32_t val, uint32_t col, uint32_t xs
 // or the raw values and norm share (a slice of a split cone).
 template <class E>
 __device__ __forceinline__ void res_tile(const ResSide& s, unsigned char* sm, E& epi, int j, uint32_t xs,
-                                         ResWs& ws, double* gout, double* gglob, uint32_t rank, uint32_t C) {
+                                         ResWs& ws, double* gout, double* gglob, double* slots, uint32_t rank, uint32_t C) {
   const int lane = threadIdx.x & 31;
   const ResTile* tp = reinterpret_cast<const ResTile*>(sm + s.o_tile) + j;
   const int rb = tp->rb, nrows = tp->nrows;
@@ -361,6 +391,7 @@ __device__ __forceinline__ void res_tile(const ResSide& s, unsigned char* sm, E&
     run_sums(val, col, xs, tp->nnz, desc, tp->nonempty, (uint32_t)__cvta_generic_to_shared(ws.acc), acc0, acc1);
   }
   Red red;
+  red_init<E::kNRed, E::kMaxMask>(red);
   if (!cone) {
     if (lane < nrows) epi.linear(rb + lane, acc0, v0, red);
     if (lane + 32 < nrows) epi.linear(rb + lane + 32, acc1, v1, red);
@@ -380,6 +411,7 @@ __device__ __forceinline__ void res_tile(const ResSide& s, unsigned char* sm, E&
     }
     const double tot = warp_sum_bcast(sq);
     if (lane == 0) s.cpart[s.big[tp->group].part_base + tp->part] = tot;
+    put_red<E>(slots, (int)rank + (int)C * j, red);
     return;
   } else {
     const ResCones& cn = reinterpret_cast<const ResCones*>(sm + s.o_cone)[j];
@@ -412,15 +444,16 @@ __device__ __forceinline__ void res_tile(const ResSide& s, unsigned char* sm, E&
     }
     __syncwarp();
   }
-  publish_rows(gout, gglob, rb, nrows, rank, C);
+  if constexpr (E::kNRed > 0) put_red<E>(slots, (int)rank + (int)C * j, red);
+  else publish_rows(gout, gglob, rb, nrows, rank, C);
 }
 
 // Projection of 64 rows of a split cone, after the barrier that follows its
 // slices: every apply tile adds the shares itself, in publish_big_norm's
 // order.
 template <class E>
-__device__ __forceinline__ void res_apply(const ResSide& s, E& epi, int t, double* gout, double* gglob, uint32_t rank,
-                                          uint32_t C) {
+__device__ __forceinline__ void res_apply(const ResSide& s, E& epi, int t, double* gout, double* gglob, double* slots,
+                                          uint32_t rank, uint32_t C) {
   const int lane = threadIdx.x & 31;
   const Task tk = s.tasks[t];
   const BigCone bc = s.big[tk.group];
@@ -441,9 +474,11 @@ __device__ __forceinline__ void res_apply(const ResSide& s, E& epi, int t, doubl
   const double tv = __ldcg(s.raw + bc.rb);
   const double ns = sqrt(warp_sum_bcast(part));
   Red red;
+  red_init<E::kNRed, E::kMaxMask>(red);
   if (lane < nrows) epi.cone_apply(tk.rb + lane, rv0, tv, ns, tk.rb + lane == bc.rb, v0, red);
   if (lane + 32 < nrows) epi.cone_apply(tk.rb + lane + 32, rv1, tv, ns, tk.rb + lane + 32 == bc.rb, v1, red);
-  publish_rows(gout, gglob, tk.rb, nrows, rank, C);
+  if constexpr (E::kNRed > 0) put_red<E>(slots, t, red);
+  else publish_rows(gout, gglob, tk.rb, nrows, rank, C);
 }
 
 template <class E>
@@ -458,22 +493,84 @@ __device__ __forceinline__ void res_stage(const RStage<E>& st, const ResArgs& a,
   gather_out(e, gout);
   e.setup(cur);
   for (int j = threadIdx.x >> 5; (int)rank + (int)C * j < s.nwork; j += kResWarps)
-    res_tile<E>(s, sm, e, j, xs, ws, gout, st.gglob, rank, C);
+    res_tile<E>(s, sm, e, j, xs, ws, gout, st.gglob, st.slots, rank, C);
+  if constexpr (E::kNRed > 0) {
+    // the split cones' own slots carry nothing (their rows' terms are the tiles')
+    if (rank == 0)
+      for (int q = threadIdx.x; q < (E::kCones ? s.nbig : s.ntasks - s.nwork + s.nbig) * kMaxRed; q += kResThreads)
+        st.slots[(int64_t)(E::kCones ? s.ntasks : s.nwork) * kMaxRed + q] = 0.0;
+  }
   if constexpr (E::kCones) {
     if (s.nbig > 0) {
       res_sync(C);
       for (int j = threadIdx.x >> 5; s.nwork + (int)rank + (int)C * j < s.ntasks; j += kResWarps)
-        res_apply<E>(s, e, s.nwork + (int)rank + (int)C * j, gout, st.gglob, rank, C);
+        res_apply<E>(s, e, s.nwork + (int)rank + (int)C * j, gout, st.gglob, st.slots, rank, C);
     }
   }
   res_sync(C);
+}
+
+// Slots in final_reduce_kernel's order (kThreads strides, then the block's
+// warps), by the first kThreads threads of one CTA; every thread calls it.
+template <class E>
+__device__ void res_final(const double* slots, int nslots, double* out, double (*s_red)[kThreads / 32]) {
+  Red r;
+  red_init<E::kNRed, E::kMaxMask>(r);
+  if (threadIdx.x < kThreads) {
+    for (int q = threadIdx.x; q < nslots; q += kThreads) {
+      Red o;
+#pragma unroll
+      for (int k = 0; k < E::kNRed; ++k) o.v[k] = __ldcg(slots + (int64_t)q * kMaxRed + k);
+      red_combine<E::kNRed, E::kMaxMask>(r, o);
+    }
+    warp_reduce<E::kNRed, E::kMaxMask>(r);
+    if ((threadIdx.x & 31) == 0)
+#pragma unroll
+      for (int k = 0; k < E::kNRed; ++k) s_red[k][threadIdx.x >> 5] = r.v[k];
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+#pragma unroll
+    for (int k = 0; k < E::kNRed; ++k) r.v[k] = s_red[k][0];
+    for (int w = 1; w < kThreads / 32; ++w) {
+      Red o;
+#pragma unroll
+      for (int k = 0; k < E::kNRed; ++k) o.v[k] = s_red[k][w];
+      red_combine<E::kNRed, E::kMaxMask>(r, o);
+    }
+#pragma unroll
+    for (int k = 0; k < E::kNRed; ++k) out[k] = r.v[k];
+  }
+  __syncthreads();
+}
+
+// The residual lanes of the batch's last (full) iterate: x_bar and y_bar
+// replace the gathered copies, and the passes of launch_residuals run over
+// the tiles that are already in shared memory.  (As separate launches the
+// check cost the host loop 50-65 us after every batch, a third of a solve at
+// n = 400: 16 checks in 150 iterations, 2.30 ms per solve before, 2.05 here.)
+__device__ void res_check(const ResCheck& k, const ResArgs& a, unsigned char* sm, const DevState* cur, ResWs& ws,
+                          uint32_t rank, uint32_t C) {
+  __shared__ double s_red[kMaxRed][kThreads / 32];
+  double* gx = reinterpret_cast<double*>(sm + k.rp.gin);
+  double* gy = reinterpret_cast<double*>(sm + k.rd.gin);
+  for (int i = threadIdx.x; i < k.n; i += kResThreads) gx[i] = __ldcg(k.x_bar + i);
+  for (int i = threadIdx.x; i < k.m; i += kResThreads) gy[i] = __ldcg(k.y_bar + i);
+  __syncthreads();
+  res_stage(k.qx, a, sm, cur, false, ws, rank, C);
+  res_stage(k.rd, a, sm, cur, false, ws, rank, C);
+  res_stage(k.rp, a, sm, cur, false, ws, rank, C);
+  if (rank == 0) {
+    res_final<EpiRd>(k.rd.slots, k.slots_x, k.out, s_red);
+    if (k.rp.on) res_final<EpiRp>(k.rp.slots, k.slots_y, k.out + 8, s_red);
+  }
 }
 
 template <class E0, class E1, class E2, class E3>
 __global__ void __launch_bounds__(kResThreads, 1)
     resident_kernel(const __grid_constant__ ResArgs a, const __grid_constant__ RStage<E0> s0,
                     const __grid_constant__ RStage<E1> s1, const __grid_constant__ RStage<E2> s2,
-                    const __grid_constant__ RStage<E3> s3) {
+                    const __grid_constant__ RStage<E3> s3, const __grid_constant__ ResCheck chk) {
   extern __shared__ __align__(16) unsigned char sm[];
   const uint32_t rank = cluster_rank(), C = cluster_size();
   ResWs& ws = reinterpret_cast<ResWs*>(sm + a.o_ws)[threadIdx.x >> 5];
@@ -496,7 +593,81 @@ __global__ void __launch_bounds__(kResThreads, 1)
     res_stage(s2, a, sm, cur, last, ws, rank, C);
     res_stage(s3, a, sm, cur, last, ws, rank, C);
   }
+  if (chk.on) res_check(chk, a, sm, st + (a.iters & 1), ws, rank, C);
   if (rank == 0 && threadIdx.x == 0) a.st->inner = inner + a.iters;
+}
+
+// Sums of NV lanes over i < n of f(i, lane sums), the same bits in every
+// thread of every CTA of the cluster.
+template <int NV, class F>
+__device__ __forceinline__ void res_sum(int n, F f, double (*s_red)[kResWarps], double* out) {
+  double v[NV];
+#pragma unroll
+  for (int k = 0; k < NV; ++k) v[k] = 0.0;
+  for (int i = threadIdx.x; i < n; i += kResThreads) f(i, v);
+#pragma unroll
+  for (int k = 0; k < NV; ++k) {
+    const double t = warp_sum_bcast(v[k]);
+    if ((threadIdx.x & 31) == 0) s_red[k][threadIdx.x >> 5] = t;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < NV; ++k) {
+    double t = 0.0;
+    for (int w = 0; w < kResWarps; ++w) t = t + s_red[k][w];
+    out[k] = t;
+  }
+  __syncthreads();
+}
+
+// The power iteration on lambda_max(AA') (power_generic's steps: q = z/|z|,
+// z = A (A' q), lambda = <q, z>, err = |z - lambda q| / (|z| + lambda)) with
+// A, A' and the vectors in the cluster's shared memory.  Every CTA holds z, q
+// and A'q in full and takes the sums itself, so only the two products need
+// the cluster.  out[0] = lambda, out[1] = iterations run.  (B200, ms per
+// estimate before / here: n = 400 1.9 / 1.07, n = 800 8.2 / 2.1, n = 2000
+// 8.2 / 2.6, n = 3000 16.5 / 5.3.)
+__global__ void __launch_bounds__(kResThreads, 1)
+    resident_power_kernel(const __grid_constant__ ResArgs a, const __grid_constant__ RStage<EpiPlain> sat,
+                          const __grid_constant__ RStage<EpiPlain> sa, const double* z0, int m, int maxit, double tol,
+                          double* out) {
+  extern __shared__ __align__(16) unsigned char sm[];
+  __shared__ double s_red[2][kResWarps];
+  const uint32_t rank = cluster_rank(), C = cluster_size();
+  ResWs& ws = reinterpret_cast<ResWs*>(sm + a.o_ws)[threadIdx.x >> 5];
+  const DevState* st = reinterpret_cast<const DevState*>(sm + a.o_state);
+  for (int i = 0; i < 2; ++i) load_side(a.side[i], sm, rank, C);
+  double* q = reinterpret_cast<double*>(sm + sat.gin);
+  double* z = reinterpret_cast<double*>(sm + sa.gout);
+  for (int i = threadIdx.x; i < m; i += kResThreads) z[i] = z0[i];
+  res_sync(C);
+  double lambda = 1.0, zz = 0.0;
+  res_sum<1>(m, [&](int i, double* v) { v[0] = v[0] + z[i] * z[i]; }, s_red, &zz);
+  int it = 0;
+  for (; it < maxit; ++it) {
+    const double nz = sqrt(zz);
+    for (int i = threadIdx.x; i < m; i += kResThreads) q[i] = z[i] / nz;
+    __syncthreads();
+    res_stage(sat, a, sm, st, false, ws, rank, C);
+    res_stage(sa, a, sm, st, false, ws, rank, C);
+    double d[2];
+    res_sum<2>(m, [&](int i, double* v) {
+      v[0] = v[0] + q[i] * z[i];
+      v[1] = v[1] + z[i] * z[i];
+    }, s_red, d);
+    lambda = d[0];
+    zz = d[1];
+    double rr;
+    res_sum<1>(m, [&](int i, double* v) {
+      const double e = z[i] - lambda * q[i];
+      v[0] = v[0] + e * e;
+    }, s_red, &rr);
+    if (sqrt(rr) / (sqrt(zz) + lambda) < tol) break;
+  }
+  if (rank == 0 && threadIdx.x == 0) {
+    out[0] = lambda;
+    out[1] = (double)it;
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -506,7 +677,7 @@ int align16(int64_t b) { return (int)((b + 15) & ~(int64_t)15); }
 
 // Shared-memory bytes of a batch on C CTAs, with the largest CTA's slots and
 // tiles per side, and the offsets (when given).
-int64_t resident_layout(const Ctx* c, const ResidentShape& r, ResArgs* a, int* goff) {
+int64_t resident_layout(const Ctx* c, const ResidentShape& r, ResArgs* a, int* goff, bool with_q) {
   int64_t o = 0;
   auto take = [&](int64_t bytes) {
     const int64_t at = o;
@@ -521,11 +692,11 @@ int64_t resident_layout(const Ctx* c, const ResidentShape& r, ResArgs* a, int* g
   // gathered vectors: y, x_hat; with Q y_bar, w (tempv in the same place: w is
   // gathered by the first half-step only), w_bar
   const int64_t len[3] = {c->m, c->n, c->n};
-  for (int k = 0; k < (c->has_q ? 3 : 2); ++k) {
+  for (int k = 0; k < (with_q ? 3 : 2); ++k) {
     const int at = take(8 * std::max<int64_t>(len[k], 1));
     if (goff) goff[k] = at;
   }
-  for (int i = 0; i < (c->has_q ? 3 : 2); ++i) {
+  for (int i = 0; i < (with_q ? 3 : 2); ++i) {
     const int ov = take(8LL * r.slots[i]), od = take(256LL * r.tiles[i]);
     const int ot = take((int64_t)sizeof(ResTile) * r.tiles[i]), oc = take((int64_t)sizeof(ResCones) * r.tiles[i]);
     const int ocol = take(2LL * r.slots[i]);
@@ -641,7 +812,7 @@ void resident_plan(Ctx* c) {
       r.slots[i] = (int)*std::max_element(used, used + C);
       r.tiles[i] = (nw + C - 1) / C;
     }
-    if (resident_layout(c, r, nullptr, nullptr) <= kResSmemMax) return;
+    if (resident_layout(c, r, nullptr, nullptr, c->has_q) <= kResSmemMax) return;
   }
 }
 
@@ -652,18 +823,13 @@ bool resident_eligible(const Ctx* c) {
                   : cluster_fits<NoQKernel>(c->device, resident_kernel<EpiX, EpiY, EpiY, EpiY>, c->res.ctas);
 }
 
-// k iterations (the last one full when full_last) in one launch.
-int launch_resident(Ctx* c, int64_t k, bool full_last) {
-  HPR_TRY(prepare_engine(c));
-  IterEpis E;
-  make_iter_epis(c, false, E);
-  ResArgs a = ResArgs();
-  int g[3] = {0, 0, 0};
-  const int64_t smem = resident_layout(c, c->res, &a, g);
+namespace {
+// The matrices and tiles of the first `ns` sides.
+void resident_sides(const Ctx* c, int ns, ResArgs& a) {
   const Plan* plans[3] = {&c->planX, &c->planY, &c->planQ};
   const int32_t* cs[3] = {c->d_var_start, c->d_con_start, c->d_var_start};
-  a.nsides = c->has_q ? 3 : 2;
-  for (int i = 0; i < a.nsides; ++i) {
+  a.nsides = ns;
+  for (int i = 0; i < ns; ++i) {
     const PlanView v = view_of(*plans[i], cs[i]);
     ResSide& s = a.side[i];
     s.tasks = v.tasks;
@@ -679,27 +845,87 @@ int launch_resident(Ctx* c, int64_t k, bool full_last) {
     s.nwork = nwork_of(*plans[i]);
     s.nbig = v.nbig;
   }
+}
+}  // namespace
+
+int launch_resident_power(Ctx* c, int maxit, double tol, double* lam, bool* done) {
+  *done = false;
+  if (c->res.ctas == 0 || c->m == 0) return HPR_OK;
+  HPR_TRY(prepare_engine(c));
+  ResArgs a = ResArgs();
+  int g[3] = {0, 0, 0};
+  // one more vector of length m (q) behind the batch's layout without Q
+  const int64_t base = resident_layout(c, c->res, &a, g, false);
+  const int64_t smem = base + 8 * c->m;
+  if (smem > kResSmemMax || !cluster_fits(c->device, resident_power_kernel, c->res.ctas)) return HPR_OK;
+  resident_sides(c, 2, a);
+  a.st = c->d_state;
+  std::vector<double> hz(c->m);
+  power_start_vector(hz, 1);
+  HPR_CUDA(c, cudaMemcpyAsync(c->pz, hz.data(), c->m * sizeof(double), cudaMemcpyHostToDevice, c->stream));
+  const RStage<EpiPlain> sat{plain(c->ptq), 0, (int)base, g[1], c->ptq, 1, nullptr};
+  const RStage<EpiPlain> sa{plain(c->pz), 1, g[1], g[0], c->pq, 1, nullptr};
+  cudaLaunchAttribute attr[1];
+  const cudaLaunchConfig_t cfg = resident_config(c->res.ctas, smem, c->stream, attr);
+  HPR_CUDA(c, cudaLaunchKernelEx(&cfg, resident_power_kernel, a, sat, sa, (const double*)c->pz, (int)c->m, maxit, tol,
+                                 c->d_red_out + 40));
+  c->launches++;
+  HPR_CUDA(c, cudaMemcpyAsync(c->h_red_out + 40, c->d_red_out + 40, 2 * sizeof(double), cudaMemcpyDeviceToHost,
+                              c->stream));
+  HPR_CUDA(c, cudaStreamSynchronize(c->stream));
+  *lam = c->h_red_out[40];
+  *done = true;
+  return HPR_OK;
+}
+
+// k iterations (the last one full when full_last) in one launch; with `check`
+// (full_last only) the residual lanes of launch_residuals too, in d_red_out.
+int launch_resident(Ctx* c, int64_t k, bool full_last, bool check) {
+  HPR_TRY(prepare_engine(c));
+  IterEpis E;
+  make_iter_epis(c, false, E);
+  ResArgs a = ResArgs();
+  int g[3] = {0, 0, 0};
+  const int64_t smem = resident_layout(c, c->res, &a, g, c->has_q);
+  resident_sides(c, c->has_q ? 3 : 2, a);
   a.st = c->d_state;
   a.g0 = c->has_q ? c->w : c->y;
   a.g0_off = c->has_q ? g[1] : g[0];
   a.g0_len = (int)(c->has_q ? c->n : c->m);
   const int hy = c->m > 0 ? 1 : 0;
+  ResCheck chk = ResCheck();
+  if (check) {
+    ResidualEpis R;
+    make_residual_epis(c, R);
+    const int gx = g[1], gy = g[0];  // x_bar in x_hat's (w's) place, y_bar in y's
+    chk.qx = {plain(c->Qx), 2, gx, g[2], c->Qx, c->has_q ? 1 : 0, nullptr};
+    chk.rd = {R.rd, 0, gy, gy, nullptr, 1, c->d_red};
+    chk.rp = {R.rp, 1, gx, gx, nullptr, hy, c->d_red + (int64_t)c->planX.nslots() * kMaxRed};
+    chk.x_bar = c->x_bar;
+    chk.y_bar = c->y_bar;
+    chk.n = (int)c->n;
+    chk.m = (int)c->m;
+    chk.slots_x = c->planX.nslots();
+    chk.slots_y = c->planY.nslots();
+    chk.out = c->d_red_out + kCheckLanes;
+  }
   cudaLaunchAttribute attr[1];
   const cudaLaunchConfig_t cfg = resident_config(c->res.ctas, smem, c->stream, attr);
   for (int64_t done = 0; done < k;) {
     a.iters = (int)std::min<int64_t>(k - done, 1 << 20);
     a.full_last = (full_last && done + a.iters == k) ? 1 : 0;
+    chk.on = check && done + a.iters == k ? 1 : 0;
     if (!c->has_q) {
-      const RStage<EpiX> sx{E.ex, 0, g[0], g[1], c->x_hat, 1};
-      const RStage<EpiY> sy{E.ey, 1, g[1], g[0], c->y, hy};
-      const RStage<EpiY> off{E.ey, 1, g[1], g[0], c->y, 0};
-      HPR_CUDA(c, cudaLaunchKernelEx(&cfg, resident_kernel<EpiX, EpiY, EpiY, EpiY>, a, sx, sy, off, off));
+      const RStage<EpiX> sx{E.ex, 0, g[0], g[1], c->x_hat, 1, nullptr};
+      const RStage<EpiY> sy{E.ey, 1, g[1], g[0], c->y, hy, nullptr};
+      const RStage<EpiY> off{E.ey, 1, g[1], g[0], c->y, 0, nullptr};
+      HPR_CUDA(c, cudaLaunchKernelEx(&cfg, resident_kernel<EpiX, EpiY, EpiY, EpiY>, a, sx, sy, off, off, chk));
     } else {
-      const RStage<EpiQX> sq{E.eq, 2, g[1], g[2], c->w_bar, 1};
-      const RStage<EpiQT> st{E.et, 2, g[2], g[1], c->tempv, hy};
-      const RStage<EpiY> sy{E.ey, 1, g[1], g[0], c->y_bar, hy};
-      const RStage<EpiW2> sw{E.e2, 0, g[0], g[1], c->w, 1};
-      HPR_CUDA(c, cudaLaunchKernelEx(&cfg, resident_kernel<EpiQX, EpiQT, EpiY, EpiW2>, a, sq, st, sy, sw));
+      const RStage<EpiQX> sq{E.eq, 2, g[1], g[2], c->w_bar, 1, nullptr};
+      const RStage<EpiQT> st{E.et, 2, g[2], g[1], c->tempv, hy, nullptr};
+      const RStage<EpiY> sy{E.ey, 1, g[1], g[0], c->y_bar, hy, nullptr};
+      const RStage<EpiW2> sw{E.e2, 0, g[0], g[1], c->w, 1, nullptr};
+      HPR_CUDA(c, cudaLaunchKernelEx(&cfg, resident_kernel<EpiQX, EpiQT, EpiY, EpiW2>, a, sq, st, sy, sw, chk));
     }
     c->launches++;
     done += a.iters;

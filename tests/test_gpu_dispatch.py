@@ -70,3 +70,25 @@ def test_resident_and_engine_agree_to_the_bit(n):
             res.append([g.get(v) for v in VECS] + [np.array(g.scalars())])
     for a, b in zip(*res):
         assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("n,kind", [(50, "none"), (400, "diag"), (1100, "none"), (2600, "none"), (1200, "csr"),
+                                    (3000, "csr")])
+def test_residual_lanes_of_a_batch_and_resident_power(n, kind):
+    """A solve's last residuals come with its last batch: they equal the
+    separate residual passes over the same iterate (same sums, 1e-13 for the
+    order of the slots).  lambda_max(AA') against the oracle's iteration."""
+    from hprsocp_b200 import Context
+    model = (instances.qp_csr(n, n=n, density=0.01) if kind == "csr"
+             else instances.small_socp(31 + n, n=n, diag_q=kind == "diag"))
+    p = HPRSOCP_parameters(verbose=False, stoptol=1e-14, max_iter=37)
+    with Context(model) as g:
+        r = g.solve(p)
+        assert r.status == "MAX_ITER" and r.iter == 37
+        again = g.residuals()
+        for k, v in r.last.items():
+            assert abs(v - again[k]) <= 1e-13 * max(1.0, abs(again[k])), (k, v, again[k])
+        o = OracleContext(model, threads=0)
+        o.scale(p)
+        assert abs(g.power_A() - o.power_A()) <= 1e-9 * o.power_A()
+        o.close()
