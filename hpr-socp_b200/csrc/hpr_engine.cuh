@@ -119,16 +119,10 @@ __device__ void block_reduce(Red& r, double (*s_red)[kThreads / 32]) {
 
 // Cache operators of the engine's loads (defaults measured best on B200:
 // gathers through L2 only, streams and epilogue inputs evict-first):
-//   gathers of xin:      0 ld.global.nc, 1 ld.global.cg (L2 only),
-//                        2 ld.global.nc.L1::no_allocate, 3 ld.global.cg with
-//                          an L2 evict-last policy;
 //   col / val streams:   0 ld.global.cs, 1 ld.global.cg,
 //                        2 ld.global.nc.L1::no_allocate with an L2 evict-first
 //                          policy, 3 ld.global.nc;
 //   epilogue inputs:     0 ld.global.cs, 1 ld.global.cg.
-#ifndef HPR_ENGINE_GATHER
-#define HPR_ENGINE_GATHER 1
-#endif
 #ifndef HPR_ENGINE_STREAM
 #define HPR_ENGINE_STREAM 0
 #endif
@@ -137,16 +131,6 @@ __device__ void block_reduce(Red& r, double (*s_red)[kThreads / 32]) {
 #endif
 
 // ---- loads with the cache operators chosen above
-__device__ __forceinline__ double ld_nc_na(const double* p) {
-  double v;
-  asm("ld.global.nc.L1::no_allocate.f64 %0, [%1];" : "=d"(v) : "l"(p));
-  return v;
-}
-__device__ __forceinline__ float ld_nc_na(const float* p) {
-  float v;
-  asm("ld.global.nc.L1::no_allocate.f32 %0, [%1];" : "=f"(v) : "l"(p));
-  return v;
-}
 __device__ __forceinline__ uint64_t l2_evict_first_policy() {
   uint64_t pol;
   asm("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(pol));
@@ -162,27 +146,12 @@ __device__ __forceinline__ double ld_stream_pol(const double* p, uint64_t pol) {
   asm("ld.global.nc.L1::no_allocate.L2::cache_hint.f64 %0, [%1], %2;" : "=d"(v) : "l"(p), "l"(pol));
   return v;
 }
-__device__ __forceinline__ uint64_t l2_evict_last_policy() {
-  uint64_t pol;
-  asm("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(pol));
-  return pol;
-}
-__device__ __forceinline__ double ld_cg_last(const double* p) {
-  double v;
-  asm("ld.global.cg.L2::cache_hint.f64 %0, [%1], %2;" : "=d"(v) : "l"(p), "l"(l2_evict_last_policy()));
-  return v;
-}
-__device__ __forceinline__ float ld_cg_last(const float* p) {
-  float v;
-  asm("ld.global.cg.L2::cache_hint.f32 %0, [%1], %2;" : "=f"(v) : "l"(p), "l"(l2_evict_last_policy()));
-  return v;
-}
-template <class T>
+// kL1: through L1 (a plain load: the vector may have been written by the kernel
+// before this one, whose end a dependent launch has waited for); else L2 only.
+template <bool kL1, class T>
 __device__ __forceinline__ T ld_gather(const T* p) {
-  if constexpr (HPR_ENGINE_GATHER == 1) return __ldcg(p);
-  else if constexpr (HPR_ENGINE_GATHER == 2) return ld_nc_na(p);
-  else if constexpr (HPR_ENGINE_GATHER == 3) return ld_cg_last(p);
-  else return __ldg(p);
+  if constexpr (kL1) return *p;
+  else return __ldcg(p);
 }
 template <class T>
 __device__ __forceinline__ T ld_stream(const T* p, uint64_t pol) {
@@ -246,8 +215,13 @@ struct EngineArgs {
 #ifndef HPR_ENGINE_MINB
 #define HPR_ENGINE_MINB 3
 #endif
+// (B200, us per iteration at 3 / 4 / 5 / 6: FP64 n = 2M 252 / 258 / 245 / 250,
+// FP32 n = 700k 98.9 / 104.7 / 102.4 / 104.4)
 #ifndef HPR_ENGINE_CHUNK
-#define HPR_ENGINE_CHUNK 4
+#define HPR_ENGINE_CHUNK 5
+#endif
+#ifndef HPR_ENGINE_CHUNK_LOW
+#define HPR_ENGINE_CHUNK_LOW 3
 #endif
 #ifndef HPR_ENGINE_PREFETCH
 #define HPR_ENGINE_PREFETCH 0  // 1: epilogue inputs loaded before the gather rounds
@@ -273,6 +247,7 @@ constexpr int kEngineThreads = kWarpsPerCta * 32;
 #endif
 constexpr int kGrab = HPR_ENGINE_GRAB;  // tiles taken per atomic
 constexpr int kChunk = HPR_ENGINE_CHUNK;  // elements per lane per gather round
+constexpr int kChunkLow = HPR_ENGINE_CHUNK_LOW;  // the same in the reduced-precision streams
 
 constexpr bool kTwoRows = kRowCap > 32;   // a lane owns rows lane and lane + 32
 
@@ -591,8 +566,8 @@ __device__ __forceinline__ void prefetch_tile(const EngineArgs& a, const Epi& ep
 // CH (U): nonzeros per lane per step.
 // pf_next >= 0: the warp's next tile, prefetched to L2 after this tile's
 // gathers.
-// kRows: the plan may hold tiles in row mode.
-template <class Epi, int PREC, bool kCoherent = false, int CH = kChunk, bool kRows = true>
+// kRows: the plan may hold tiles in row mode.  kL1: gathers through L1.
+template <class Epi, int PREC, bool kCoherent = false, int CH = kChunk, bool kRows = true, bool kL1 = false>
 __device__ void process_warp_tile(const EngineArgs& a, Epi& epi, int tix, WarpSmem& ws, int pf_next = -1) {
   constexpr int U = CH;
   const int lane = threadIdx.x & 31;
@@ -672,9 +647,9 @@ __device__ void process_warp_tile(const EngineArgs& a, Epi& epi, int tix, WarpSm
         p[u] = 0.0;
         if (k0 + u < my) {
           if constexpr (PREC == HPR_PREC_FP64)
-            p[u] = vals[u] * (kCoherent ? __ldcg(a.xin + cols[u]) : ld_gather(a.xin + cols[u]));
+            p[u] = vals[u] * (kCoherent ? __ldcg(a.xin + cols[u]) : ld_gather<kL1>(a.xin + cols[u]));
           else
-            p[u] = (double)((float)vals[u] * (kCoherent ? __ldcg(a.xin32 + cols[u]) : ld_gather(a.xin32 + cols[u])));
+            p[u] = (double)((float)vals[u] * (kCoherent ? __ldcg(a.xin32 + cols[u]) : ld_gather<kL1>(a.xin32 + cols[u])));
         }
       }
       if (!HPR_ENGINE_PIPE && k0 + U < R) load_step(k0 + U, ncols, nvals);
@@ -792,9 +767,9 @@ template <class Epi>
 struct EngineMinBlocks {
   static constexpr int value = HPR_ENGINE_MINB;
 };
-template <class Epi>
+template <class Epi, int PREC>
 struct EngineChunk {
-  static constexpr int value = kChunk;
+  static constexpr int value = PREC == HPR_PREC_FP64 ? kChunk : kChunkLow;
 };
 
 // kStatic (host-chosen, only for plans without split cones): first tiles by
@@ -818,10 +793,10 @@ struct EngineChunk {
 // tile per warp the third CTA hides more latency: n = 2M 262 / 269.)
 constexpr int kWideBlocks = 2;
 constexpr int kWideChunk = 8;
-template <class Epi, int PREC, bool kStatic, bool kWide>
+template <class Epi, int PREC, bool kStatic, bool kWide, bool kL1>
 __global__ void __launch_bounds__(kEngineThreads, kWide ? kWideBlocks : EngineMinBlocks<Epi>::value)
     engine_kernel(EngineArgs a, Epi epi) {
-  constexpr int kCh = kWide ? kWideChunk : EngineChunk<Epi>::value;
+  constexpr int kCh = kWide ? kWideChunk : EngineChunk<Epi, PREC>::value;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   WarpSmem* s_ws = reinterpret_cast<WarpSmem*>(smem_raw);
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -844,7 +819,7 @@ __global__ void __launch_bounds__(kEngineThreads, kWide ? kWideBlocks : EngineMi
     }
     while (base < ntasks) {
       for (int q = 0; q < kGrab && base + q < ntasks; ++q)
-        process_warp_tile<Epi, PREC, false, kCh, kWide>(a, epi, base + q, ws);
+        process_warp_tile<Epi, PREC, false, kCh, kWide, kL1>(a, epi, base + q, ws);
       int next = ntasks;
       if (dyn && lane == 0) next = nstat + atomicAdd(a.pv.task_ctr, kGrab);
       base = __shfl_sync(0xffffffffu, next, 0);
@@ -864,7 +839,7 @@ __global__ void __launch_bounds__(kEngineThreads, kWide ? kWideBlocks : EngineMi
           pf = __shfl_sync(0xffffffffu, next, 0);
           pf = pf < ntasks ? pf : -1;
         }
-        process_warp_tile<Epi, PREC, false, kCh, kWide>(a, epi, base + q, ws, pf);
+        process_warp_tile<Epi, PREC, false, kCh, kWide, kL1>(a, epi, base + q, ws, pf);
       }
       if (!HPR_ENGINE_EARLYGRAB && lane == 0) next = atomicAdd(a.pv.task_ctr, kGrab);
       base = __shfl_sync(0xffffffffu, next, 0);

@@ -216,8 +216,8 @@ struct EpiQX {
 };
 // (the Q path's x-step holds more state per row: two nonzeros per lane per
 // round keep it from spilling)
-template <>
-struct EngineChunk<EpiQX> {
+template <int PREC>
+struct EngineChunk<EpiQX, PREC> {
   static constexpr int value = kChunk < 2 ? kChunk : 2;
 };
 

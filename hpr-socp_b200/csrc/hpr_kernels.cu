@@ -232,14 +232,14 @@ namespace {
 
 // Persistent grid size of one engine instantiation (resident CTAs per SM x
 // SMs), computed once.
-template <class Epi, int PREC, bool kStatic, bool kWide>
+template <class Epi, int PREC, bool kStatic, bool kWide, bool kL1>
 int engine_grid(int* smem_bytes) {
   static std::once_flag once;
   static int grid = 1;
   constexpr int dyn = kEngineSmem;
   *smem_bytes = dyn;
   std::call_once(once, [] {
-    auto k = engine_kernel<Epi, PREC, kStatic, kWide>;
+    auto k = engine_kernel<Epi, PREC, kStatic, kWide, kL1>;
     cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn);
     // (the kWide form keeps the other form's carveout: an SM drains before it
     // changes its carveout, which cost the Q path's mixed launches 3.4 of 136 us)
@@ -257,10 +257,10 @@ int engine_grid(int* smem_bytes) {
 
 // One warp per tile at most: a small problem occupies only the SMs it needs,
 // so other streams (other contexts of a serving process) run beside it.
-template <class Epi, int PREC, bool kStatic, bool kWide>
+template <class Epi, int PREC, bool kStatic, bool kWide, bool kL1>
 void launch_engine_form(Ctx* c, int nt, const EngineArgs& a, const Epi& epi) {
   int dyn = 0;
-  const int full = engine_grid<Epi, PREC, kStatic, kWide>(&dyn);
+  const int full = engine_grid<Epi, PREC, kStatic, kWide, kL1>(&dyn);
   const int g = std::max(1, std::min(full, (nt + kWarpsPerCta - 1) / kWarpsPerCta));
 #if HPR_ENGINE_PDL
   // programmatic dependent launch: the kernel may be scheduled while the
@@ -276,11 +276,22 @@ void launch_engine_form(Ctx* c, int nt, const EngineArgs& a, const Epi& epi) {
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  cudaLaunchKernelEx(&cfg, engine_kernel<Epi, PREC, kStatic, kWide>, a, epi);
+  cudaLaunchKernelEx(&cfg, engine_kernel<Epi, PREC, kStatic, kWide, kL1>, a, epi);
 #else
-  engine_kernel<Epi, PREC, kStatic, kWide><<<g, kEngineThreads, dyn, c->stream>>>(a, epi);
+  engine_kernel<Epi, PREC, kStatic, kWide, kL1><<<g, kEngineThreads, dyn, c->stream>>>(a, epi);
 #endif
 }
+
+// Gathers from a vector of up to this many entries go through L1: where rows'
+// columns are near one another (or, as in F'(F w), the vector is short) lines
+// are found there.  Measured on B200, us per iteration with L2-only gathers /
+// through L1: the Q path at n = 200k 136.1 / 102.8; uniformly random columns,
+// which find nothing, 55.4 / 55.4 at n = 300k, 97.7 / 98.0 at 700k, 153.0 /
+// 154.1 at 1.2M, 246.0 / 248.4 at 2M.
+#ifndef HPR_GATHER_L1_MAX
+#define HPR_GATHER_L1_MAX (1 << 20)
+#endif
+constexpr int64_t kGatherL1Max = HPR_GATHER_L1_MAX;
 
 // tiles of one wave of the kWide form: one per warp, two CTAs per SM
 int engine_wide_tiles() {
@@ -301,12 +312,15 @@ int engine_wide_tiles() {
 template <class Epi, int PREC>
 void launch_engine_prec(Ctx* c, int nt, const EngineArgs& a, const Epi& epi) {
   const bool wide = nt <= engine_wide_tiles();
+  const bool l1 = a.M.ncols <= kGatherL1Max;
   if (a.pv.nbig == 0) {
-    if (wide) launch_engine_form<Epi, PREC, true, true>(c, nt, a, epi);
-    else launch_engine_form<Epi, PREC, true, false>(c, nt, a, epi);
+    if (wide) launch_engine_form<Epi, PREC, true, true, true>(c, nt, a, epi);
+    else if (l1) launch_engine_form<Epi, PREC, true, false, true>(c, nt, a, epi);
+    else launch_engine_form<Epi, PREC, true, false, false>(c, nt, a, epi);
   } else {
-    if (wide) launch_engine_form<Epi, PREC, false, true>(c, nt, a, epi);
-    else launch_engine_form<Epi, PREC, false, false>(c, nt, a, epi);
+    if (wide) launch_engine_form<Epi, PREC, false, true, true>(c, nt, a, epi);
+    else if (l1) launch_engine_form<Epi, PREC, false, false, true>(c, nt, a, epi);
+    else launch_engine_form<Epi, PREC, false, false, false>(c, nt, a, epi);
   }
 }
 

@@ -92,3 +92,10 @@ def test_residual_lanes_of_a_batch_and_resident_power(n, kind):
         o.scale(p)
         assert abs(g.power_A() - o.power_A()) <= 1e-9 * o.power_A()
         o.close()
+
+
+@pytest.mark.parametrize("scale", [0.52, 0.53])
+def test_gathers_through_l1_and_past_it(scale):
+    """1,040,000 and 1,060,000 columns: both sides of the line (2^20) below
+    which the gathers go through L1."""
+    _check(instances.config1(6, scale=scale), iters=3)
