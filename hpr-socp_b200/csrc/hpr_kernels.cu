@@ -358,7 +358,8 @@ int engine_launch(Ctx* c, const DevCSR& M, const Plan& p, const int32_t* cone_st
     if (wide_reduce && ns > 2 * kThreads && c->d_red2) {
       // two fixed-order levels: contiguous chunks of slots per CTA, then
       // the chunk sums (one CTA reading tens of thousands of slots is a
-      // tenth of a power-iteration step on the benchmark)
+      // tenth of a power-iteration step on the benchmark; 58 + 50 us of the
+      // residual check's 390 there)
       const int g = std::min<int>(kWideReduceCtas, (ns + kThreads - 1) / kThreads);
       slot_chunk_kernel<Epi::kNRed, Epi::kMaxMask><<<g, kThreads, 0, c->stream>>>(c->d_red, ns, c->d_red2);
       final_reduce_kernel<Epi::kNRed, Epi::kMaxMask><<<1, kThreads, 0, c->stream>>>(c->d_red2, g,
@@ -713,28 +714,51 @@ __global__ void bounds_box_kernel(int64_t n, const double* l, const double* u, c
     dx[i] = (lv + uv) * (bs / col[i]);
   }
 }
-// compute_err_soc_kernel! (kernels.jl:6617-6655)
+// compute_err_soc_kernel! (kernels.jl:6617-6655).  A warp per cone, the lanes
+// striding over its rows (one thread per cone read a 5000-row cone alone: 2.34
+// ms of a re-solve at n = 2M and 0.6 ms at n = 100k, 20 us here); cones of up
+// to kSerialCone rows are taken 32 at a time, one per lane.
+constexpr int kSerialCone = 8;
+__device__ __forceinline__ void bounds_row(int64_t j, bool head, double t, double ns, const double* xb,
+                                           const double* col, double bs, double* dx) {
+  double v = xb[j];
+  if (ns <= -t) {
+  } else if (ns <= t) {
+    v = 0.0;
+  } else {
+    const double f = (1 + t / ns) / 2;
+    v = head ? (ns + t) / 2 - t : f * v - v;
+  }
+  dx[j] = v * (bs / col[j]);
+}
 __global__ void bounds_cone_kernel(int64_t ncones, const int32_t* vs, const double* xb, const double* col, double bs,
                                    double* dx) {
-  for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < ncones; k += (int64_t)gridDim.x * blockDim.x) {
-    int64_t st = vs[k], en = vs[k + 1];
-    double t = xb[st];
-    double ns = 0.0;
-    dx[st] = t;
-    for (int64_t j = st + 1; j < en; ++j) {
-      dx[j] = xb[j];
-      ns += xb[j] * xb[j];
+  const int lane = threadIdx.x & 31;
+  const int64_t w = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
+  for (int64_t k0 = 32 * w; k0 < ncones; k0 += 32 * nw) {
+    const int64_t k = k0 + lane;
+    const int32_t st = k < ncones ? vs[k] : 0, en = k < ncones ? vs[k + 1] : 0;
+    const bool big = en - st > kSerialCone;
+    if (!big && en > st) {
+      const double t = xb[st];
+      double ns = 0.0;
+      for (int32_t j = st + 1; j < en; ++j) ns += xb[j] * xb[j];
+      ns = sqrt(ns);
+      for (int32_t j = st; j < en; ++j) bounds_row(j, j == st, t, ns, xb, col, bs, dx);
     }
-    ns = sqrt(ns);
-    if (ns <= -t) {
-    } else if (ns <= t) {
-      for (int64_t j = st; j < en; ++j) dx[j] = 0.0;
-    } else {
-      double f = (1 + t / ns) / 2;
-      dx[st] = (ns + t) / 2 - t;
-      for (int64_t j = st + 1; j < en; ++j) dx[j] = f * dx[j] - dx[j];
+    unsigned todo = __ballot_sync(0xffffffffu, big);
+    while (todo) {
+      const int src = __ffs((int)todo) - 1;
+      todo &= todo - 1;
+      const int32_t b = __shfl_sync(0xffffffffu, st, src), e = __shfl_sync(0xffffffffu, en, src);
+      const double t = xb[b];
+      double ns = 0.0;
+#pragma unroll 4
+      for (int32_t j = b + 1 + lane; j < e; j += 32) ns += xb[j] * xb[j];
+      ns = sqrt(warp_sum_bcast(ns));
+      for (int32_t j = b + lane; j < e; j += 32) bounds_row(j, j == b, t, ns, xb, col, bs, dx);
     }
-    for (int64_t j = st; j < en; ++j) dx[j] *= bs / col[j];
   }
 }
 }  // namespace
@@ -746,8 +770,8 @@ int launch_residuals(Ctx* c, bool include_bounds, hpr_residuals* r) {
   if (!skipq) HPR_TRY(qmap(c, c->x_bar, c->Qx, c->ftmp));
   ResidualEpis R;
   make_residual_epis(c, R);
-  HPR_TRY(engine_launch(c, c->AT, c->planX, c->d_var_start, c->y_bar, nullptr, R.rd, false, true, 0));
-  if (c->m > 0) HPR_TRY(engine_launch(c, c->A, c->planY, c->d_con_start, c->x_bar, nullptr, R.rp, false, true, 8));
+  HPR_TRY(engine_launch(c, c->AT, c->planX, c->d_var_start, c->y_bar, nullptr, R.rd, false, true, 0, true));
+  if (c->m > 0) HPR_TRY(engine_launch(c, c->A, c->planY, c->d_con_start, c->x_bar, nullptr, R.rp, false, true, 8, true));
   if (include_bounds) {
     bounds_box_kernel<<<592, kThreads, 0, c->stream>>>(c->n, c->l, c->u, c->x_bar, c->col_norm, bs, c->dx);
     int64_t nv = (int64_t)c->h_var_idx.size() - 1;
@@ -808,7 +832,7 @@ int launch_mnorm(Ctx* c, double* out) {
     EpiDot e{};
     e.lin_src[0] = e.cone_src[0] = c->dx;
     e.out = c->ATdy;
-    HPR_TRY(engine_launch(c, c->AT, c->planX, c->d_var_start, c->dy, nullptr, e, false, true, 2));
+    HPR_TRY(engine_launch(c, c->AT, c->planX, c->d_var_start, c->dy, nullptr, e, false, true, 2, true));
   }
   HPR_TRY(fetch_red(c, 8));
   for (int k = 0; k < 5; ++k) h[k] = c->h_red_out[k];
