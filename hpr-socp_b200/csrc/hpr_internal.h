@@ -379,9 +379,15 @@ int h2d_copy(Ctx* c, void* dst, const void* src, size_t bytes);
 // the same for an array of doubles, checked on the way (check 1: every
 // value finite, 2: no NaN); *ok is false if a value fails
 int h2d_copy_checked(Ctx* c, void* dst, const void* src, size_t bytes, int check, bool* ok);
-// device-to-host copy into a pageable host array after the work enqueued on
-// the context's stream; returns once the data is in dst
-int d2h_copy(Ctx* c, void* dst, const void* src, size_t bytes);
+// device-to-host copies into pageable host arrays (dst2: a second copy, or
+// null) after the work enqueued on the context's stream; returns once the data
+// is there
+struct HostCopy {
+  void *dst, *dst2;
+  const void* src;
+  size_t bytes;
+};
+int d2h_copy(Ctx* c, const HostCopy* copies, int n);
 // pred(v[i]) for every i, checked on several host threads for long arrays
 bool host_all(const double* v, int64_t n, bool (*pred)(double));
 // Runs f on a new thread added to `pool`, or on the calling thread when no

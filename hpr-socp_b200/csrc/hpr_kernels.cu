@@ -11,6 +11,7 @@
 #include <mutex>
 #include <set>
 #include <string>
+#include <vector>
 
 #include "hpr_epilogues.cuh"
 
@@ -1295,27 +1296,31 @@ int launch_unscale(Ctx* c, double* hx, double* hy, double* hz, double* hw) {
   const double bs = c->b_scale, cs = c->c_scale;
   const double *xb = c->x_bar, *col = c->col_norm, *zb = c->z_bar, *wb = c->w_bar, *yb = c->y_bar,
                *row = c->row_norm;
-  double* t = c->vtmp_n;
-  size_t nb = (size_t)c->n * sizeof(double);
+  // every vector into a work vector of its own, then one read-back of all
+  const size_t nb = (size_t)c->n * sizeof(double), mb = (size_t)c->m * sizeof(double);
+  std::vector<HostCopy> out;
   if (hx || (hw && !c->has_q)) {
+    double* t = c->vtmp_n;
     HPR_TRY(vec_map(c, c->n, [=] __device__(int64_t i) { t[i] = bs * (xb[i] / col[i]); }));
-    if (hx) HPR_TRY(d2h_copy(c, hx, t, nb));
-    if (hw && !c->has_q) HPR_TRY(d2h_copy(c, hw, t, nb));
+    double* w = c->has_q ? nullptr : hw;  // without Q w is x
+    out.push_back({hx ? hx : w, hx ? w : nullptr, t, nb});
   }
   if (hw && c->has_q) {
+    double* t = c->tempv;
     HPR_TRY(vec_map(c, c->n, [=] __device__(int64_t i) { t[i] = bs * (wb[i] / col[i]); }));
-    HPR_TRY(d2h_copy(c, hw, t, nb));
+    out.push_back({hw, nullptr, t, nb});
   }
   if (hz) {
+    double* t = c->Rd;
     HPR_TRY(vec_map(c, c->n, [=] __device__(int64_t i) { t[i] = cs * (zb[i] * col[i]); }));
-    HPR_TRY(d2h_copy(c, hz, t, nb));
+    out.push_back({hz, nullptr, t, nb});
   }
   if (hy && c->m > 0) {
-    double* tm = c->vtmp_m;
-    HPR_TRY(vec_map(c, c->m, [=] __device__(int64_t i) { tm[i] = cs * (yb[i] / row[i]); }));
-    HPR_TRY(d2h_copy(c, hy, tm, (size_t)c->m * sizeof(double)));
+    double* t = c->vtmp_m;
+    HPR_TRY(vec_map(c, c->m, [=] __device__(int64_t i) { t[i] = cs * (yb[i] / row[i]); }));
+    out.push_back({hy, nullptr, t, mb});
   }
-  return HPR_OK;
+  return d2h_copy(c, out.data(), (int)out.size());
 }
 
 // process_initial_points! (algorithm.jl:2612-2677)
@@ -1324,7 +1329,7 @@ int launch_initial_points(Ctx* c, const double* hx0, const double* hy0) {
   const int64_t n = c->n, m = c->m;
   const bool hq = c->has_q;
   if (hx0) {
-    HPR_CUDA(c, cudaMemcpyAsync(c->vtmp_n, hx0, n * sizeof(double), cudaMemcpyHostToDevice, c->stream));
+    HPR_TRY(h2d_copy(c, c->vtmp_n, hx0, n * sizeof(double)));
     const double *t = c->vtmp_n, *col = c->col_norm;
     double *x = c->x, *xb = c->x_bar, *lx = c->last_x, *w = c->w, *wb = c->w_bar, *lw = c->last_w;
     HPR_TRY(vec_map(c, n, [=] __device__(int64_t i) {
@@ -1340,7 +1345,7 @@ int launch_initial_points(Ctx* c, const double* hx0, const double* hy0) {
     }));
   }
   if (hy0) {
-    HPR_CUDA(c, cudaMemcpyAsync(c->vtmp_m, hy0, m * sizeof(double), cudaMemcpyHostToDevice, c->stream));
+    HPR_TRY(h2d_copy(c, c->vtmp_m, hy0, m * sizeof(double)));
     const double *t = c->vtmp_m, *row = c->row_norm;
     double *y = c->y, *yb = c->y_bar, *ly = c->last_y;
     HPR_TRY(vec_map(c, m, [=] __device__(int64_t i) {

@@ -153,6 +153,7 @@ constexpr int kStageThreads = 8;
 constexpr int kStageSlots = 2;
 constexpr size_t kStageChunk = (size_t)4 << 20;
 constexpr size_t kStageMin = (size_t)4 << 20;  // smaller copies go straight to cudaMemcpyAsync
+constexpr size_t kStageRead = (size_t)1 << 20;   // a read-back's chunk
 constexpr int kStageDevices = 64;
 
 struct Stage {
@@ -258,49 +259,65 @@ int h2d_copy_checked(Ctx* c, void* dst, const void* src, size_t bytes, int check
   return HPR_OK;
 }
 
-int d2h_copy(Ctx* c, void* dst, const void* src, size_t bytes) {
-  if (bytes == 0) return HPR_OK;
-  if (bytes < kStageMin || c->device < 0 || c->device >= kStageDevices) {
-    HPR_CUDA(c, cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, c->stream));
+int d2h_copy(Ctx* c, const HostCopy* copies, int n) {
+  size_t total = 0;
+  for (int k = 0; k < n; ++k) total += copies[k].bytes;
+  if (total == 0) return HPR_OK;
+  auto plain = [&]() {
+    for (int k = 0; k < n; ++k)
+      if (copies[k].bytes)
+        HPR_CUDA(c, cudaMemcpyAsync(copies[k].dst, copies[k].src, copies[k].bytes, cudaMemcpyDeviceToHost, c->stream));
     HPR_CUDA(c, cudaStreamSynchronize(c->stream));
+    for (int k = 0; k < n; ++k)
+      if (copies[k].bytes && copies[k].dst2) std::memcpy(copies[k].dst2, copies[k].dst, copies[k].bytes);
     return HPR_OK;
-  }
+  };
+  if (total < kStageMin || c->device < 0 || c->device >= kStageDevices) return plain();
   Stage& st = g_stage[c->device];
   std::lock_guard<std::mutex> lock(st.mu);
-  if (!stage_init(st, c->device)) {
-    HPR_CUDA(c, cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, c->stream));
-    HPR_CUDA(c, cudaStreamSynchronize(c->stream));
-    return HPR_OK;
-  }
-  const size_t nchunks = (bytes + kStageChunk - 1) / kStageChunk;
+  if (!stage_init(st, c->device)) return plain();
+  // chunks over all the arrays; thread t moves chunks t, t + nt, ...
+  struct Chunk {
+    const HostCopy* h;
+    size_t off, len;
+  };
+  std::vector<Chunk> chunks;
+  for (int k = 0; k < n; ++k)
+    for (size_t o = 0; o < copies[k].bytes; o += kStageRead)
+      chunks.push_back({copies + k, o, std::min(kStageRead, copies[k].bytes - o)});
+  const size_t nchunks = chunks.size();
+  const int nt = (int)std::min<size_t>(kStageThreads, nchunks);
   std::atomic<int> err{0};
-  // thread t moves chunks t, t + kStageThreads, ...: the chunk's DMA into
-  // its pinned slot, then (once that DMA is done) the host copy out of it
+  // the next chunk's DMA runs into one pinned slot while the host copies the
+  // chunk before it out of the other
   auto worker = [&](int t) {
     if (cudaSetDevice(c->device) != cudaSuccess) {
       err.store(1);
       return;
     }
-    int use = 0;
-    for (size_t k = (size_t)t; k < nchunks && !err.load(); k += kStageThreads, use ^= 1) {
-      const size_t off = k * kStageChunk;
-      const size_t len = std::min(kStageChunk, bytes - off);
-      if (st.used[t][use] && cudaEventSynchronize(st.ev[t][use]) != cudaSuccess) {
-        err.store(1);
-        return;
-      }
-      if (cudaMemcpyAsync(st.buf[t][use], static_cast<const char*>(src) + off, len, cudaMemcpyDeviceToHost,
+    auto start = [&](size_t k, int use) {
+      const Chunk& h = chunks[k];
+      if ((st.used[t][use] && cudaEventSynchronize(st.ev[t][use]) != cudaSuccess) ||
+          cudaMemcpyAsync(st.buf[t][use], static_cast<const char*>(h.h->src) + h.off, h.len, cudaMemcpyDeviceToHost,
                           c->stream) != cudaSuccess ||
-          cudaEventRecord(st.ev[t][use], c->stream) != cudaSuccess ||
-          cudaEventSynchronize(st.ev[t][use]) != cudaSuccess) {
+          cudaEventRecord(st.ev[t][use], c->stream) != cudaSuccess)
+        err.store(1);
+      else
+        st.used[t][use] = true;
+    };
+    int use = 0;
+    if ((size_t)t < nchunks) start((size_t)t, use);
+    for (size_t k = (size_t)t; k < nchunks && !err.load(); k += nt, use ^= 1) {
+      if (k + nt < nchunks) start(k + nt, use ^ 1);
+      if (err.load() || cudaEventSynchronize(st.ev[t][use]) != cudaSuccess) {
         err.store(1);
         return;
       }
-      st.used[t][use] = true;
-      std::memcpy(static_cast<char*>(dst) + off, st.buf[t][use], len);
+      const Chunk& h = chunks[k];
+      std::memcpy(static_cast<char*>(h.h->dst) + h.off, st.buf[t][use], h.len);
+      if (h.h->dst2) std::memcpy(static_cast<char*>(h.h->dst2) + h.off, st.buf[t][use], h.len);
     }
   };
-  const int nt = (int)std::min<size_t>(kStageThreads, nchunks);
   std::vector<std::thread> th;
   for (int t = 1; t < nt; ++t) spawn_or_run(th, [&worker, t] { worker(t); });
   worker(0);
