@@ -566,8 +566,8 @@ __device__ __forceinline__ void prefetch_tile(const EngineArgs& a, const Epi& ep
 // CH (U): nonzeros per lane per step.
 // pf_next >= 0: the warp's next tile, prefetched to L2 after this tile's
 // gathers.
-// kRows: the plan may hold tiles in row mode.  kL1: gathers through L1.
-template <class Epi, int PREC, bool kCoherent = false, int CH = kChunk, bool kRows = true, bool kL1 = false>
+// kL1: gathers through L1.
+template <class Epi, int PREC, bool kCoherent = false, int CH = kChunk, bool kL1 = false>
 __device__ void process_warp_tile(const EngineArgs& a, Epi& epi, int tix, WarpSmem& ws, int pf_next = -1) {
   constexpr int U = CH;
   const int lane = threadIdx.x & 31;
@@ -590,12 +590,11 @@ __device__ void process_warp_tile(const EngineArgs& a, Epi& epi, int tix, WarpSm
   const int nnz = tp->nze - tp->nzb;
   const uint64_t desc = a.pv.desc[(int64_t)tix * 32 + lane];
   const TileRun* rp = a.pv.runs + tix;
-  const bool rows = kRows && rp->r0 >= 0;  // row mode: the lane's rows, one after the other
-  int R = rows ? rp->r0 : (nnz + 31) >> 5;
+  const int R = (nnz + 31) >> 5;
   int my = nnz - lane * R;
-  my = rows ? (int)(desc & 0xffff) : (my < 0 ? 0 : (my > R ? R : my));
+  my = my < 0 ? 0 : (my > R ? R : my);
   const uint64_t pol = HPR_ENGINE_STREAM == 2 ? l2_evict_first_policy() : 0;
-  const uint32_t heads = rows ? 0u : (uint32_t)desc;
+  const uint32_t heads = (uint32_t)desc;
   const int j0 = (int)(desc >> kDescOrdShift);
   double acc0 = 0.0, acc1 = 0.0;  // sums of rows rb + lane and rb + lane + 32
   Vals<Epi::kSlots> v0, v1;
@@ -608,12 +607,12 @@ __device__ void process_warp_tile(const EngineArgs& a, Epi& epi, int tix, WarpSm
   }
 
   // ---- 1. products, added per lane in column order
-  int64_t base = (int64_t)rp->sbase + lane;
+  const int64_t base = (int64_t)rp->sbase + lane;
   double s = 0.0;
   const uint32_t acc = smem_addr(ws.acc);
   uint32_t next = acc + 8 * j0;                  // slot of the next row to start (by non-empty ordinal)
   uint32_t close = acc + 8 * (kRowCap + lane);   // where the segment being summed goes
-  for (int h = 0;; ++h) {
+  {
     // one base address per array and step; the U loads of a step sit at
     // fixed offsets from it
     auto load_step = [&](int k0, int32_t* cc, double* vv) {
@@ -677,20 +676,9 @@ __device__ void process_warp_tile(const EngineArgs& a, Epi& epi, int tix, WarpSm
         vals[u] = nvals[u];
       }
     }
-    if constexpr (!kRows) break;
-    if (!rows) break;
-    if (h > 0 || rp->r1 == 0) {
-      (h > 0 ? acc1 : acc0) = s;
-      break;
-    }
-    acc0 = s;
-    s = 0.0;
-    base += 32 * (int64_t)R;
-    R = rp->r1;
-    my = (int)((desc >> 16) & 0xffff);
   }
-  if (!rows && my > 0) sts_f64(close, s);
-  const double cont = !rows && my > 0 ? lds_f64(acc + 8 * (kRowCap + lane)) : 0.0;
+  if (my > 0) sts_f64(close, s);
+  const double cont = my > 0 ? lds_f64(acc + 8 * (kRowCap + lane)) : 0.0;
 
   if (HPR_ENGINE_L2PF >= 2 && pf_next >= 0) prefetch_tile<Epi, PREC>(a, epi, pf_next);
   const Task t = *tp;
@@ -713,7 +701,7 @@ __device__ void process_warp_tile(const EngineArgs& a, Epi& epi, int tix, WarpSm
 
   // ---- 2. continuations: segmented scan over the lanes, then added to the
   // row's head segment
-  if (!rows) {
+  {
     const bool has_cont = my > 0 && !(heads & 1u);
     const int key = has_cont ? j0 - 1 : -2 - lane;
     double v = has_cont ? cont : 0.0;
@@ -733,7 +721,7 @@ __device__ void process_warp_tile(const EngineArgs& a, Epi& epi, int tix, WarpSm
   }
 
   // ---- 3. row sums to the owning lanes (empty rows sum to zero)
-  if (!rows) {
+  {
     const unsigned lt = (1u << lane) - 1u;
     const uint64_t ne = rp->nonempty;
     const unsigned b0 = (unsigned)(ne & 0xffffffffull);
@@ -783,8 +771,7 @@ struct EngineChunk {
 // B200: the static form is 3-4% faster on the Q path's short launches and
 // 0.5% slower on the benchmark's long ones, so each plan gets its form.)
 //
-// kWide (host-chosen, plans of at most one tile per warp at two CTAs per SM;
-// plans with row-mode tiles are always of that size):
+// kWide (host-chosen, plans of at most one tile per warp at two CTAs per SM):
 // a launch then lasts as long as one tile's chain, and more warps per SM
 // cannot shorten it; two CTAs per SM leave 128 registers per thread, so
 // eight nonzeros per lane are in flight and nothing spills.  (Measured on
@@ -819,7 +806,7 @@ __global__ void __launch_bounds__(kEngineThreads, kWide ? kWideBlocks : EngineMi
     }
     while (base < ntasks) {
       for (int q = 0; q < kGrab && base + q < ntasks; ++q)
-        process_warp_tile<Epi, PREC, false, kCh, kWide, kL1>(a, epi, base + q, ws);
+        process_warp_tile<Epi, PREC, false, kCh, kL1>(a, epi, base + q, ws);
       int next = ntasks;
       if (dyn && lane == 0) next = nstat + atomicAdd(a.pv.task_ctr, kGrab);
       base = __shfl_sync(0xffffffffu, next, 0);
@@ -839,7 +826,7 @@ __global__ void __launch_bounds__(kEngineThreads, kWide ? kWideBlocks : EngineMi
           pf = __shfl_sync(0xffffffffu, next, 0);
           pf = pf < ntasks ? pf : -1;
         }
-        process_warp_tile<Epi, PREC, false, kCh, kWide, kL1>(a, epi, base + q, ws, pf);
+        process_warp_tile<Epi, PREC, false, kCh, kL1>(a, epi, base + q, ws, pf);
       }
       if (!HPR_ENGINE_EARLYGRAB && lane == 0) next = atomicAdd(a.pv.task_ctr, kGrab);
       base = __shfl_sync(0xffffffffu, next, 0);

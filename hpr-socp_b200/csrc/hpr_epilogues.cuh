@@ -590,8 +590,7 @@ inline void make_residual_epis(Ctx* c, ResidualEpis& R) {
 #define HPR_FUSED_MAX_TILES (4 * kWarpsPerCta)
 #endif
 constexpr int kFusedMaxTiles = HPR_FUSED_MAX_TILES;
-// (soft caps cut a full tile into about four)
-inline bool one_cta_plan(const Plan& p) { return (int64_t)p.tasks.size() <= (p.soft ? 4 : 1) * kFusedMaxTiles; }
+inline bool one_cta_plan(const Plan& p) { return (int64_t)p.tasks.size() <= kFusedMaxTiles; }
 #ifndef HPR_FUSED_CHUNK
 #define HPR_FUSED_CHUNK 8
 #endif

@@ -70,25 +70,12 @@ static_assert(sizeof(Task) == 32, "Task layout");
 // k: a non-empty row begins at run element k) and, from bit kDescOrdShift,
 // the number of non-empty rows that begin in runs 0..L-1.  `nonempty` marks the tile's
 // non-empty rows (bit r for row rb + r).
-//
-// A tile in row mode (r0 >= 0; only plans with soft caps have them) gives each
-// lane whole rows instead: element k of row rb + lane at slot
-// sbase + 32 k + lane (r0 steps, the longest such row) and element k of row
-// rb + 32 + lane at slot sbase + 32 (r0 + k) + lane (r1 steps); `desc` holds
-// the two rows' lengths (16 bits each).  A row is then summed by one lane in
-// column order with no row starts and no sums across lanes; it is chosen
-// where the longest rows take no more than kRowModeSteps steps beyond R (a
-// step of runs costs about twice a step of rows, and the sums across lanes a
-// fixed amount) and at most about a third of the slots are padding.
 struct TileRun {
   uint64_t nonempty;
   int32_t sbase;
   int32_t soff;  // cluster-resident batches: first slot in the owning CTA's shared memory
-  int32_t r0, r1;
-  int64_t pad;
 };
-static_assert(sizeof(TileRun) == 32, "TileRun layout");
-constexpr int kRowModeSteps = 12;
+static_assert(sizeof(TileRun) == 16, "TileRun layout");
 constexpr int kDescOrdShift = 32;
 static_assert(kNnzTile <= 32 * kDescOrdShift, "a run's row-start bits must fit below kDescOrdShift");
 
@@ -117,7 +104,6 @@ struct Plan {
   std::vector<TileRun> runs;   // per tile (run layout)
   std::vector<uint64_t> desc;  // per tile and lane (run layout)
   int64_t tslots = 0;          // slots of the tiled arrays (nonzeros + run padding)
-  bool soft = false;           // built with soft caps (several tiles where a full tile would do)
   // device copies
   Task* d_tasks = nullptr;
   BigCone* d_big = nullptr;
@@ -151,15 +137,10 @@ struct Plan {
 // of every cone plus an end sentinel (empty when the side has no cones);
 // rows before cone_starts[0] are linear rows.
 // `nnz_cap` (<= kNnzTile; 0: kNnzTile) caps the nonzeros of a tile.
-// `soft_nnz` / `soft_rows` (0: none) end a tile of linear rows, of small
-// cones or of a split cone's slice early, without splitting a row or a small
-// cone that fits the hard caps.
 void build_plan(const std::vector<int32_t>& rowptr, int64_t nrows,
-                const std::vector<int64_t>& cone_starts, Plan& plan, int nnz_cap = 0, int soft_nnz = 0,
-                int soft_rows = 0);
-// the run layout of the plan's tiles (called by build_plan), in row mode where
-// that is shorter and row_mode allows it
-void build_runs(const std::vector<int32_t>& rowptr, Plan& plan, bool row_mode = false);
+                const std::vector<int64_t>& cone_starts, Plan& plan, int nnz_cap = 0);
+// the run layout of the plan's tiles (called by build_plan)
+void build_runs(const std::vector<int32_t>& rowptr, Plan& plan);
 
 struct DevCSR {
   int64_t nrows = 0, ncols = 0, nnz = 0;
@@ -211,10 +192,10 @@ struct PlanView {
 };
 
 // Cluster-resident batches (hpr_resident.cu): CTAs of the cluster (0: the
-// problem does not fit), soft tile caps, and the largest CTA's slots and
-// tiles per side (A', A, Q).
+// problem does not fit) and the largest CTA's slots and tiles per side (A', A,
+// Q).
 struct ResidentShape {
-  int ctas = 0, soft_nnz = 0, soft_rows = 0;
+  int ctas = 0;
   int slots[3] = {0, 0, 0}, tiles[3] = {0, 0, 0};
 };
 
@@ -341,7 +322,6 @@ int run_iterations(Ctx* c, int64_t k, bool full_last, bool check = false, bool* 
 // (then no partial-iteration graph is captured)
 bool uses_fused_iterations(const Ctx* c);
 // cluster-resident batches (hpr_resident.cu)
-ResidentShape resident_estimate(int64_t m, int64_t n, int64_t nnz, int64_t qnnz, bool has_q);
 void resident_plan(Ctx* c);  // after the plans are built, before upload_plan
 bool resident_eligible(const Ctx* c);
 int launch_resident(Ctx* c, int64_t k, bool full_last, bool check);

@@ -111,8 +111,7 @@ PlanView view_of(const Plan& p, const int32_t* cone_start) {
 // ---------------------------------------------------------------------------
 namespace {
 template <class T>
-__global__ void tile_layout_kernel(const Task* __restrict__ tasks, const TileRun* __restrict__ runs,
-                                   const uint64_t* __restrict__ desc, int ntasks,
+__global__ void tile_layout_kernel(const Task* __restrict__ tasks, const TileRun* __restrict__ runs, int ntasks,
                                    const int32_t* __restrict__ col, const T* __restrict__ val,
                                    int32_t* __restrict__ tcol, T* __restrict__ tval) {
   const int lane = threadIdx.x & 31;
@@ -123,27 +122,6 @@ __global__ void tile_layout_kernel(const Task* __restrict__ tasks, const TileRun
     const int32_t nnz = t.nze - t.nzb;
     const int32_t R = (nnz + 31) / 32;
     const int64_t sb = runs[ti].sbase;
-    if (runs[ti].r0 >= 0) {
-      // row mode: a lane's rows start at the sum of the rows before them
-      const uint64_t d = desc[ti * 32 + lane];
-      int32_t start = t.nzb;
-      for (int h = 0; h < 2; ++h) {
-        const int32_t len = (int32_t)((d >> (16 * h)) & 0xffff), steps = h ? runs[ti].r1 : runs[ti].r0;
-        int32_t inc = len;
-        for (int o = 1; o < 32; o <<= 1) {
-          const int32_t v = __shfl_up_sync(0xffffffffu, inc, o);
-          if (lane >= o) inc += v;
-        }
-        const int64_t s0 = sb + 32 * (int64_t)(h ? runs[ti].r0 : 0) + lane;
-        for (int32_t k = 0; k < steps; ++k) {
-          const int32_t e = start + inc - len + k;
-          if (tcol) tcol[s0 + 32 * k] = k < len ? col[e] : 0;
-          tval[s0 + 32 * k] = k < len ? val[e] : T(0.0f);
-        }
-        start += __shfl_sync(0xffffffffu, inc, 31);
-      }
-      continue;
-    }
     for (int32_t k = 0; k < R; ++k) {
       const int32_t e = lane * R + k;  // element k of this lane's run
       const int64_t d = sb + 32 * (int64_t)k + lane;
@@ -163,7 +141,7 @@ int tile_layout(Ctx* c, const Plan& p, const int32_t* col, const T* val, int32_t
   const int nt = (int)p.tasks.size();
   if (nt == 0) return HPR_OK;
   const int blocks = std::min(148 * 8, (nt + 7) / 8);
-  tile_layout_kernel<T><<<blocks, 256, 0, c->stream>>>(p.d_tasks, p.d_runs, p.d_desc, nt, col, val, tcol, tval);
+  tile_layout_kernel<T><<<blocks, 256, 0, c->stream>>>(p.d_tasks, p.d_runs, nt, col, val, tcol, tval);
   c->launches++;
   HPR_CUDA(c, cudaGetLastError());
   return HPR_OK;

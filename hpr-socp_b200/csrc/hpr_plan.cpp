@@ -58,10 +58,8 @@ void emit_long_row(const std::vector<int32_t>& rp, int32_t r, int32_t bigslot,
 }  // namespace
 
 void build_plan(const std::vector<int32_t>& rp, int64_t nrows,
-                const std::vector<int64_t>& cone_starts, Plan& plan, int nnz_cap, int soft_nnz, int soft_rows) {
+                const std::vector<int64_t>& cone_starts, Plan& plan, int nnz_cap) {
   const int32_t cap = (nnz_cap > 0 && nnz_cap < kNnzTile) ? nnz_cap : kNnzTile;
-  const int64_t snnz = (soft_nnz > 0 && soft_nnz < cap) ? soft_nnz : cap;
-  const int64_t srows = (soft_rows > 0 && soft_rows < kRowCap) ? soft_rows : kRowCap;
   plan.nrows = nrows;
   plan.tasks.clear();
   plan.big.clear();
@@ -75,10 +73,10 @@ void build_plan(const std::vector<int32_t>& rp, int64_t nrows,
   int64_t r = 0;
   while (r < lin_end) {
     int64_t start = r, cnt = 0, nz = 0;
-    while (r < lin_end && cnt < srows) {
+    while (r < lin_end && cnt < kRowCap) {
       int64_t rn = (int64_t)rp[r + 1] - rp[r];
       if (rn > cap) break;
-      if (nz + rn > snnz && cnt > 0) break;
+      if (nz + rn > cap && cnt > 0) break;
       nz += rn;
       cnt++;
       r++;
@@ -116,8 +114,8 @@ void build_plan(const std::vector<int32_t>& rp, int64_t nrows,
     bool big = d > kSmallConeMax || cnz > cap;
     if (d <= 0) continue;
     if (!big) {
-      if (open && ((cur.re - cur.rb) + d > srows ||
-                   (int64_t)(cur.nze - cur.nzb) + cnz > snnz ||
+      if (open && ((cur.re - cur.rb) + d > kRowCap ||
+                   (int64_t)(cur.nze - cur.nzb) + cnz > cap ||
                    cur.ncones >= 32000))
         flush();
       if (!open) {
@@ -155,10 +153,10 @@ void build_plan(const std::vector<int32_t>& rp, int64_t nrows,
         continue;
       }
       int64_t start = q, cnt = 0, nz = 0;
-      while (q < b && cnt < srows) {
+      while (q < b && cnt < kRowCap) {
         int64_t rq = (int64_t)rp[q + 1] - rp[q];
         if (rq > cap) break;
-        if (nz + rq > snnz && cnt > 0) break;
+        if (nz + rq > cap && cnt > 0) break;
         nz += rq;
         cnt++;
         q++;
@@ -210,13 +208,12 @@ void build_plan(const std::vector<int32_t>& rp, int64_t nrows,
       bc.napply++;
     }
   }
-  plan.soft = soft_nnz > 0;
-  build_runs(rp, plan, plan.soft);
+  build_runs(rp, plan);
 }
 
 // Run layout of every tile (TileRun): slot offsets, non-empty rows and the
 // per-lane row-start descriptors.
-void build_runs(const std::vector<int32_t>& rp, Plan& plan, bool row_mode) {
+void build_runs(const std::vector<int32_t>& rp, Plan& plan) {
   const size_t nt = plan.tasks.size();
   plan.runs.assign(nt, TileRun{});
   plan.desc.assign(nt * 32, 0u);
@@ -227,23 +224,6 @@ void build_runs(const std::vector<int32_t>& rp, Plan& plan, bool row_mode) {
     const int32_t R = (nnz + 31) / 32;
     TileRun& tr = plan.runs[ti];
     tr.sbase = (int32_t)std::min<int64_t>(slots, INT32_MAX);
-    tr.r0 = tr.r1 = -1;
-    if (row_mode && t.kind != TASK_LONG_PART && t.kind != TASK_CONE_APPLY) {
-      int32_t len[2] = {0, 0};
-      for (int32_t q = t.rb; q < t.re; ++q)
-        len[(q - t.rb) / 32] = std::max(len[(q - t.rb) / 32], rp[q + 1] - rp[q]);
-      if (len[0] + len[1] <= R + kRowModeSteps && 32 * (len[0] + len[1]) <= nnz + nnz / 2 + 128) {
-        tr.r0 = len[0];
-        tr.r1 = len[1];
-        slots += 32 * (int64_t)(len[0] + len[1]);
-        for (int32_t q = t.rb; q < t.re; ++q) {
-          const int32_t n = rp[q + 1] - rp[q], r = q - t.rb;
-          if (n > 0) tr.nonempty |= 1ull << r;
-          plan.desc[ti * 32 + r % 32] |= (uint64_t)n << (r < 32 ? 0 : 16);
-        }
-        continue;
-      }
-    }
     slots += 32 * (int64_t)R;
     if (t.kind == TASK_LONG_PART) {
       tr.nonempty = 1;  // one row; its runs carry no row starts

@@ -5,9 +5,10 @@
 // record, columns, gathers, epilogue inputs, stores) and of instructions, not
 // bytes.  Measured on B200, us per iteration of a 150-iteration batch, before
 // (single-CTA kernel through L2 up to n = 400, else the multi-CTA engine) and
-// here: n = 61 5.7 / 3.7, n = 400 12.0 / 7.1, n = 800 22 / 10.6, the same with
-// a diagonal Q 25.6 / 14.4, n = 2000 27.6 / 14.7, n = 3000 with a general CSR
-// Q 30 / 14.8.  What is left is mostly the row sums' and cones' chains.
+// here: n = 61 5.7 / 4.1, n = 400 12.0 / 7.4, n = 800 22 / 12.2, the same with
+// a diagonal Q 25.6 / 15.3, n = 2000 27.6 / 13.6, n = 3000 with a general CSR
+// Q 30 / 16.2.  What is left is the instruction chain of a tile: row sums,
+// cone norms, projections.
 // Here every CTA of one cluster copies its share of the matrices (columns as
 // 16 bits, values in FP64, in the engine's run layout) and the tile records
 // into shared memory once per batch and keeps a full copy of each gathered
@@ -21,8 +22,10 @@
 // Sums, projections and their order are the engine's (hpr_engine.cuh), so the
 // iterates are the engine's to the bit.
 #include <algorithm>
+#include <map>
 #include <mutex>
 #include <set>
+#include <tuple>
 #include <vector>
 
 #include "hpr_epilogues.cuh"
@@ -44,9 +47,8 @@ struct ResTile {
   uint64_t nonempty;
   int16_t kind, ncones;
   int32_t cone, group, part;
-  int32_t r0, r1;
 };
-static_assert(sizeof(ResTile) == 48, "ResTile layout");
+static_assert(sizeof(ResTile) == 40, "ResTile layout");
 
 // cone layout of a tile of whole cones: row of each row's cone head, first
 // row of each cone (+ end)
@@ -168,9 +170,13 @@ __device__ __forceinline__ void gather_out(EpiY& e, double* p) {
   else e.y = p;
 }
 __device__ __forceinline__ void gather_out(EpiPlain& e, double* p) { e.out = p; }
+__device__ __forceinline__ void gather_out(EpiScale& e, double* p) { e.out = p; }
+__device__ __forceinline__ void gather_out(EpiPow& e, double* p) { e.out = p; }
 __device__ __forceinline__ void gather_out(EpiRd&, double*) {}
 __device__ __forceinline__ void gather_out(EpiRp&, double*) {}
 __device__ __forceinline__ void set_full(EpiPlain&, int) {}
+__device__ __forceinline__ void set_full(EpiScale&, int) {}
+__device__ __forceinline__ void set_full(EpiPow&, int) {}
 __device__ __forceinline__ void set_full(EpiRd&, int) {}
 __device__ __forceinline__ void set_full(EpiRp&, int) {}
 __device__ __forceinline__ void set_full(EpiX& e, int f) { e.full = f; }
@@ -217,8 +223,6 @@ __device__ void load_side(const ResSide& s, unsigned char* sm, uint32_t rank, ui
       x.nrows = tk.re - tk.rb;
       x.nnz = tk.nze - tk.nzb;
       x.soff = tr.soff;
-      x.r0 = tr.r0;
-      x.r1 = tr.r1;
       x.nonempty = tr.nonempty;
       x.kind = tk.kind;
       x.ncones = tk.ncones;
@@ -234,16 +238,12 @@ __device__ void load_side(const ResSide& s, unsigned char* sm, uint32_t rank, ui
       if (k == tk.ncones - 1) cones[j].start[k + 1] = (uint8_t)c1;
       for (int r = c0; r < c1; ++r) cones[j].head[r] = (uint8_t)c0;
     }
-    // the tile's steps (row mode: of its first and second 32 rows), each
-    // group padded with zeros
-    const int n0 = tr.r0 >= 0 ? tr.r0 : (tk.nze - tk.nzb + 31) >> 5, n1 = tr.r0 >= 0 ? tr.r1 : 0;
-    const int p0 = pad_steps(n0), all = p0 + pad_steps(n1);
+    // the tile's steps, the last group padded with zeros
+    const int steps = (tk.nze - tk.nzb + 31) >> 5, all = pad_steps(steps);
 #pragma unroll 4
     for (int k = 0; k < all; ++k) {
-      const int g = k < p0 ? k : n0 + k - p0;  // step in the plan's arrays
-      const bool in = k < p0 ? k < n0 : k - p0 < n1;
-      val[tr.soff + 32 * k + lane] = in ? __ldcs(s.tval + tr.sbase + 32 * g + lane) : 0.0;
-      col[tr.soff + 32 * k + lane] = in ? (uint16_t)__ldcs(s.tcol + tr.sbase + 32 * g + lane) : (uint16_t)0;
+      val[tr.soff + 32 * k + lane] = k < steps ? __ldcs(s.tval + tr.sbase + 32 * k + lane) : 0.0;
+      col[tr.soff + 32 * k + lane] = k < steps ? (uint16_t)__ldcs(s.tcol + tr.sbase + 32 * k + lane) : (uint16_t)0;
     }
   }
 }
@@ -267,34 +267,11 @@ __device__ __forceinline__ void publish_rows(double* gout, double* gglob, int rb
   }
 }
 
-// Sum of one row per lane (row mode): `steps` slots (padded to whole groups of
-// kResUnroll), the lane's own row has `len` of them.  The loads are not
-// conditional (padding is value 0, column 0, its product not used): a branch
-// around each load made every nonzero wait for the one before it.
-__device__ __forceinline__ double row_sum(uint32_t val, uint32_t col, uint32_t xs, int steps, int len) {
-  double sum = 0.0;
-  for (int k0 = 0; k0 < steps; k0 += kResUnroll) {
-    uint32_t c[kResUnroll];
-    double v[kResUnroll], x[kResUnroll];
-#pragma unroll
-    for (int u = 0; u < kResUnroll; ++u) {
-      c[u] = lds_u16(col + 64 * u);
-      v[u] = lds_f64(val + 256 * u);
-    }
-#pragma unroll
-    for (int u = 0; u < kResUnroll; ++u) x[u] = lds_f64(xs + 8 * c[u]);
-#pragma unroll
-    for (int u = 0; u < kResUnroll; ++u) {
-      const double q = v[u] * x[u];
-      sum = sum + (k0 + u < len ? q : 0.0);
-    }
-    col += 64 * kResUnroll;
-    val += 256 * kResUnroll;
-  }
-  return sum;
-}
-
-// Row sums of a tile in runs (process_warp_tile's steps 1 to 3).
+// Row sums of a tile (process_warp_tile's steps 1 to 3).  The loads are not
+// conditional (padding is value 0, column 0, and its product is not used): a
+// branch around each load made every nonzero wait for the one before it (n =
+// 400: 9.9 us per iteration against 8.3), and generic pointers cost more
+// instructions than 32-bit shared addresses (8.3 against 7.2).
 __device__ __forceinline__ void run_sums(uint32_t val, uint32_t col, uint32_t xs, int nnz, uint64_t desc,
                                          uint64_t nonempty, uint32_t acc, double& acc0, double& acc1) {
   const int lane = threadIdx.x & 31;
@@ -380,16 +357,7 @@ __device__ __forceinline__ void res_tile(const ResSide& s, unsigned char* sm, E&
   const uint32_t smb = (uint32_t)__cvta_generic_to_shared(sm);
   const uint32_t val = smb + s.o_val + 8 * (tp->soff + lane), col = smb + s.o_col + 2 * (tp->soff + lane);
   double acc0 = 0.0, acc1 = 0.0;  // sums of rows rb + lane and rb + lane + 32
-  const int r0 = tp->r0;
-  if (r0 >= 0) {
-    // row mode: the lane's rows, in column order
-    acc0 = row_sum(val, col, xs, r0, (int)(desc & 0xffff));
-    const int r1 = tp->r1;
-    const int o1 = 32 * pad_steps(r0);
-    if (r1 > 0) acc1 = row_sum(val + 8 * o1, col + 2 * o1, xs, r1, (int)((desc >> 16) & 0xffff));
-  } else {
-    run_sums(val, col, xs, tp->nnz, desc, tp->nonempty, (uint32_t)__cvta_generic_to_shared(ws.acc), acc0, acc1);
-  }
+  run_sums(val, col, xs, tp->nnz, desc, tp->nonempty, (uint32_t)__cvta_generic_to_shared(ws.acc), acc0, acc1);
   Red red;
   red_init<E::kNRed, E::kMaxMask>(red);
   if (!cone) {
@@ -444,8 +412,8 @@ __device__ __forceinline__ void res_tile(const ResSide& s, unsigned char* sm, E&
     }
     __syncwarp();
   }
-  if constexpr (E::kNRed > 0) put_red<E>(slots, (int)rank + (int)C * j, red);
-  else publish_rows(gout, gglob, rb, nrows, rank, C);
+  put_red<E>(slots, (int)rank + (int)C * j, red);
+  if (gglob) publish_rows(gout, gglob, rb, nrows, rank, C);
 }
 
 // Projection of 64 rows of a split cone, after the barrier that follows its
@@ -477,8 +445,8 @@ __device__ __forceinline__ void res_apply(const ResSide& s, E& epi, int t, doubl
   red_init<E::kNRed, E::kMaxMask>(red);
   if (lane < nrows) epi.cone_apply(tk.rb + lane, rv0, tv, ns, tk.rb + lane == bc.rb, v0, red);
   if (lane + 32 < nrows) epi.cone_apply(tk.rb + lane + 32, rv1, tv, ns, tk.rb + lane + 32 == bc.rb, v1, red);
-  if constexpr (E::kNRed > 0) put_red<E>(slots, t, red);
-  else publish_rows(gout, gglob, tk.rb, nrows, rank, C);
+  put_red<E>(slots, t, red);
+  if (gglob) publish_rows(gout, gglob, tk.rb, nrows, rank, C);
 }
 
 template <class E>
@@ -597,76 +565,110 @@ __global__ void __launch_bounds__(kResThreads, 1)
   if (rank == 0 && threadIdx.x == 0) a.st->inner = inner + a.iters;
 }
 
-// Sums of NV lanes over i < n of f(i, lane sums), the same bits in every
-// thread of every CTA of the cluster.
+// Sums of NV lanes over i < n of f(i, lane sums), in the order of a block of
+// kThreads threads (block_reduce), the same bits in every thread of every CTA.
 template <int NV, class F>
-__device__ __forceinline__ void res_sum(int n, F f, double (*s_red)[kResWarps], double* out) {
-  double v[NV];
+__device__ __forceinline__ void res_sum(int n, F f, double (*s_red)[kThreads / 32], double* out) {
+  if (threadIdx.x < kThreads) {
+    Red r;
+    red_init<NV, 0>(r);
+    for (int i = threadIdx.x; i < n; i += kThreads) f(i, r);
+    warp_reduce<NV, 0>(r);
+    if ((threadIdx.x & 31) == 0)
 #pragma unroll
-  for (int k = 0; k < NV; ++k) v[k] = 0.0;
-  for (int i = threadIdx.x; i < n; i += kResThreads) f(i, v);
-#pragma unroll
-  for (int k = 0; k < NV; ++k) {
-    const double t = warp_sum_bcast(v[k]);
-    if ((threadIdx.x & 31) == 0) s_red[k][threadIdx.x >> 5] = t;
+      for (int k = 0; k < NV; ++k) s_red[k][threadIdx.x >> 5] = r.v[k];
   }
   __syncthreads();
 #pragma unroll
   for (int k = 0; k < NV; ++k) {
-    double t = 0.0;
-    for (int w = 0; w < kResWarps; ++w) t = t + s_red[k][w];
+    double t = s_red[k][0];
+    for (int w = 1; w < kThreads / 32; ++w) t = t + s_red[k][w];
     out[k] = t;
   }
   __syncthreads();
 }
 
-// The power iteration on lambda_max(AA') (power_generic's steps: q = z/|z|,
-// z = A (A' q), lambda = <q, z>, err = |z - lambda q| / (|z| + lambda)) with
-// A, A' and the vectors in the cluster's shared memory.  Every CTA holds z, q
-// and A'q in full and takes the sums itself, so only the two products need
-// the cluster.  out[0] = lambda, out[1] = iterations run.  (B200, ms per
-// estimate before / here: n = 400 1.9 / 1.07, n = 800 8.2 / 2.1, n = 2000
-// 8.2 / 2.6, n = 3000 16.5 / 5.3.)
+// The power iteration on lambda_max(AA') with A, A' and the vectors in the
+// cluster's shared memory, in the arithmetic of the kernels it stands for, to
+// the bit: fused_power_kernel (kTwoPass false: q = z/|z|, z = A (A' q), lambda
+// = <q, z>, err = |z - lambda q| / (|z| + lambda); every CTA holds z and q in
+// full and takes the sums itself, so only the products need the cluster) and
+// power_two_pass_A (kTwoPass: the norm folded into the first product and the
+// sums taken by the second product's tiles).  out[0] = lambda, out[1] =
+// iterations run.  (B200, ms per estimate before / here: n = 400 1.9 / 1.1,
+// n = 800 8.2 / 2.5, n = 2000 8.2 / 2.6, n = 3000 16.5 / 5.5.)
+struct ResPower {
+  double *z, *z2;         // iterates in global memory (z: the start vector)
+  const double* nz2;      // kTwoPass: |z|^2 of the start vector
+  double *lanes, *out;
+  int m, maxit, slots;
+  double tol;
+};
+template <bool kTwoPass>
 __global__ void __launch_bounds__(kResThreads, 1)
     resident_power_kernel(const __grid_constant__ ResArgs a, const __grid_constant__ RStage<EpiPlain> sat,
-                          const __grid_constant__ RStage<EpiPlain> sa, const double* z0, int m, int maxit, double tol,
-                          double* out) {
+                          const __grid_constant__ RStage<EpiPlain> sa, const __grid_constant__ RStage<EpiScale> ss,
+                          const __grid_constant__ RStage<EpiPow> sp, const __grid_constant__ ResPower p) {
   extern __shared__ __align__(16) unsigned char sm[];
-  __shared__ double s_red[2][kResWarps];
+  __shared__ double s_red[kMaxRed][kThreads / 32];
+  __shared__ double s_nz2;
   const uint32_t rank = cluster_rank(), C = cluster_size();
   ResWs& ws = reinterpret_cast<ResWs*>(sm + a.o_ws)[threadIdx.x >> 5];
   const DevState* st = reinterpret_cast<const DevState*>(sm + a.o_state);
   for (int i = 0; i < 2; ++i) load_side(a.side[i], sm, rank, C);
-  double* q = reinterpret_cast<double*>(sm + sat.gin);
+  const int m = p.m;
   double* z = reinterpret_cast<double*>(sm + sa.gout);
-  for (int i = threadIdx.x; i < m; i += kResThreads) z[i] = z0[i];
+  for (int i = threadIdx.x; i < m; i += kResThreads) z[i] = p.z[i];
+  if (kTwoPass && threadIdx.x == 0) s_nz2 = *p.nz2;
   res_sync(C);
-  double lambda = 1.0, zz = 0.0;
-  res_sum<1>(m, [&](int i, double* v) { v[0] = v[0] + z[i] * z[i]; }, s_red, &zz);
+  double lambda = 1.0;
   int it = 0;
-  for (; it < maxit; ++it) {
-    const double nz = sqrt(zz);
-    for (int i = threadIdx.x; i < m; i += kResThreads) q[i] = z[i] / nz;
-    __syncthreads();
-    res_stage(sat, a, sm, st, false, ws, rank, C);
-    res_stage(sa, a, sm, st, false, ws, rank, C);
-    double d[2];
-    res_sum<2>(m, [&](int i, double* v) {
-      v[0] = v[0] + q[i] * z[i];
-      v[1] = v[1] + z[i] * z[i];
-    }, s_red, d);
-    lambda = d[0];
-    zz = d[1];
-    double rr;
-    res_sum<1>(m, [&](int i, double* v) {
-      const double e = z[i] - lambda * q[i];
-      v[0] = v[0] + e * e;
-    }, s_red, &rr);
-    if (sqrt(rr) / (sqrt(zz) + lambda) < tol) break;
+  if constexpr (kTwoPass) {
+    double nz2 = s_nz2;
+    while (it < p.maxit) {
+      RStage<EpiScale> s1 = ss;
+      s1.e.nz2 = &s_nz2;
+      res_stage(s1, a, sm, st, false, ws, rank, C);
+      RStage<EpiPow> s2 = sp;
+      s2.e.lin_src[0] = (it & 1) ? p.z2 : p.z;
+      s2.gglob = (it & 1) ? p.z : p.z2;
+      res_stage(s2, a, sm, st, false, ws, rank, C);
+      if (rank == 0) res_final<EpiPow>(sp.slots, p.slots, p.lanes, s_red);
+      res_sync(C);
+      const double nn2 = __ldcg(p.lanes), dot = __ldcg(p.lanes + 1);
+      lambda = dot / sqrt(nz2);
+      const double r2 = cmax(nn2 - lambda * lambda, 0.0);
+      const double err = sqrt(r2) / (sqrt(nn2) + lambda);
+      nz2 = nn2;
+      ++it;
+      if (err < p.tol) break;
+      if (threadIdx.x == 0) s_nz2 = nn2;
+      res_sync(C);
+    }
+  } else {
+    double* q = reinterpret_cast<double*>(sm + sat.gin);
+    double zz = 0.0;
+    res_sum<1>(m, [&](int i, Red& r) { r.v[0] = r.v[0] + z[i] * z[i]; }, s_red, &zz);
+    for (; it < p.maxit; ++it) {
+      const double nz = sqrt(zz);
+      for (int i = threadIdx.x; i < m; i += kResThreads) q[i] = z[i] / nz;
+      __syncthreads();
+      res_stage(sat, a, sm, st, false, ws, rank, C);
+      res_stage(sa, a, sm, st, false, ws, rank, C);
+      res_sum<1>(m, [&](int i, Red& r) { r.v[0] = r.v[0] + q[i] * z[i]; }, s_red, &lambda);
+      double d[2];
+      res_sum<2>(m, [&](int i, Red& r) {
+        const double e = z[i] - lambda * q[i];
+        r.v[0] = r.v[0] + e * e;
+        r.v[1] = r.v[1] + z[i] * z[i];
+      }, s_red, d);
+      zz = d[1];
+      if (sqrt(d[0]) / (sqrt(zz) + lambda) < p.tol) break;
+    }
   }
   if (rank == 0 && threadIdx.x == 0) {
-    out[0] = lambda;
-    out[1] = (double)it;
+    p.out[0] = lambda;
+    p.out[1] = (double)it;
   }
 }
 
@@ -717,9 +719,6 @@ int nwork_of(const Plan& p) {
   return n;
 }
 
-using NoQKernel = decltype(&resident_kernel<EpiX, EpiY, EpiY, EpiY>);
-using QKernel = decltype(&resident_kernel<EpiQX, EpiQT, EpiY, EpiW2>);
-
 cudaLaunchConfig_t resident_config(int C, int64_t smem, cudaStream_t stream, cudaLaunchAttribute* attr) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)C);
@@ -740,90 +739,81 @@ cudaLaunchConfig_t resident_config(int C, int64_t smem, cudaStream_t stream, cud
 template <class K>
 bool cluster_fits(int device, K kernel, int C) {
   static std::mutex mu;
-  static std::set<int> ready;                    // devices whose attributes are set
-  static std::set<std::pair<int, int>> yes, no;  // (device, CTAs)
+  static std::set<std::pair<int, const void*>> ready;              // (device, kernel) whose attributes are set
+  static std::map<std::tuple<int, const void*, int>, bool> known;  // (device, kernel, CTAs)
   std::lock_guard<std::mutex> lk(mu);
-  if (yes.count({device, C})) return true;
-  if (no.count({device, C})) return false;
-  if (!ready.count(device)) {
+  const void* id = (const void*)kernel;
+  const auto it = known.find({device, id, C});
+  if (it != known.end()) return it->second;
+  if (!ready.count({device, id})) {
     if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kResSmemMax) != cudaSuccess ||
         cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
       (void)cudaGetLastError();
       return false;
     }
-    ready.insert(device);
+    ready.insert({device, id});
   }
   cudaLaunchAttribute attr[1];
   const cudaLaunchConfig_t cfg = resident_config(C, kResSmemMax, nullptr, attr);
   int n = 0;
   const bool ok = cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) == cudaSuccess && n > 0;
   if (!ok) (void)cudaGetLastError();
-  (ok ? yes : no).insert({device, C});
+  known[{device, id, C}] = ok;
   return ok;
 }
 
 }  // namespace
 
-// The cluster size for a problem of these sizes and the soft tile caps that
-// spread its rows over the cluster's warps (0 CTAs: does not fit).  The
-// smallest cluster that holds the problem: a larger one spreads the same
-// chains over more barriers (measured on B200, us per iteration on 1 / 2 / 4 /
-// 8 / 16 CTAs: n = 61 4.3 / 5.3 / 5.1 / 5.2 / 5.1, n = 400 9.9 / 10.5 / 10.2 /
-// 10.3 / 10.9), and the other SMs serve other contexts.
-ResidentShape resident_estimate(int64_t m, int64_t n, int64_t nnz, int64_t qnnz, bool has_q) {
-  ResidentShape r;
-  if (n > 65536 || m > 65536 || n == 0) return r;
-  const int64_t gather = 8 * (m + n + (has_q ? n : 0));
-  for (int C = 1; C <= kResMaxCtas; C *= 2) {
-    const int64_t warps = (int64_t)C * kResWarps;
-    const int64_t cap = std::min<int64_t>((nnz * 5 / 4 / warps + 127) / 128 * 128, kNnzTile);
-    const int64_t tiles = 3 * kResWarps;  // about one per warp and side (resident_plan has the exact sizes)
-    const int64_t bytes = gather + (2 * nnz + qnnz) / C * 11 + tiles * 440 + kResWarps * (int64_t)sizeof(ResWs) + 2048;
-    if (bytes > kResSmemMax) continue;
-    r.ctas = C;
-    r.soft_nnz = (int)std::max<int64_t>(cap, 128);
-    r.soft_rows = 32;  // one row per lane
-    return r;
-  }
-  return r;
-}
-
-// Slot offsets of the plans' tiles in their CTA's shared memory (TileRun.pad)
-// for the cluster size of c->res, raised until the batch fits; c->res.ctas
-// becomes 0 when it does not (or a side has a row longer than a tile).
+// The cluster size for the context's problem and the slot offsets of its plans'
+// tiles in their CTA's shared memory (TileRun.soff).  c->res.ctas is 0 when the
+// problem does not fit the largest cluster or a side has a row longer than a
+// tile.  The smallest cluster that holds it is taken: a larger one only adds
+// barriers to the same chains (measured on B200, us per iteration on 1 / 2 / 4 /
+// 8 / 16 CTAs with an earlier form of the sums: n = 61 4.3 / 5.3 / 5.1 / 5.2 /
+// 5.1, n = 400 9.9 / 10.5 / 10.2 / 10.3 / 10.9), and the other SMs serve other
+// contexts.
 void resident_plan(Ctx* c) {
-  ResidentShape& r = c->res;
+  c->res = ResidentShape();
+  ResidentShape r;
+  if (c->n > 65536 || c->m > 65536 || (c->q_kind != HPR_Q_NONE && c->q_kind != HPR_Q_CSR)) return;
   Plan* plans[3] = {&c->planX, &c->planY, &c->planQ};
   const int ns = c->has_q ? 3 : 2;
   for (int i = 0; i < ns; ++i)
-    if (!plans[i]->lng.empty()) r.ctas = 0;
-  for (; r.ctas > 0; r.ctas = r.ctas < kResMaxCtas ? 2 * r.ctas : 0) {
+    if (!plans[i]->lng.empty()) return;
+  if (plans[0]->tasks.empty() || (c->A.nnz + c->Q.nnz) / kResMaxCtas * 20 > kResSmemMax) return;
+  for (r.ctas = 1; r.ctas <= kResMaxCtas; r.ctas *= 2) {
     const int C = r.ctas;
     for (int i = 0; i < ns; ++i) {
       Plan& p = *plans[i];
       int64_t used[kResMaxCtas] = {0};
       const int nw = nwork_of(p);
       for (int t = 0; t < nw; ++t) {
-        TileRun& tr = p.runs[t];
-        tr.soff = (int32_t)used[t % C];
-        used[t % C] += 32 * (int64_t)(tr.r0 >= 0 ? pad_steps(tr.r0) + pad_steps(tr.r1)
-                                                 : pad_steps((p.tasks[t].nze - p.tasks[t].nzb + 31) / 32));
+        p.runs[t].soff = (int32_t)used[t % C];
+        used[t % C] += 32 * (int64_t)pad_steps((p.tasks[t].nze - p.tasks[t].nzb + 31) / 32);
       }
       r.slots[i] = (int)*std::max_element(used, used + C);
       r.tiles[i] = (nw + C - 1) / C;
     }
-    if (resident_layout(c, r, nullptr, nullptr, c->has_q) <= kResSmemMax) return;
+    if (resident_layout(c, r, nullptr, nullptr, c->has_q) <= kResSmemMax) {
+      c->res = r;
+      return;
+    }
   }
 }
 
 bool resident_eligible(const Ctx* c) {
   if (c->res.ctas == 0 || c->precision != HPR_PREC_FP64) return false;
   if (c->q_kind != HPR_Q_NONE && c->q_kind != HPR_Q_CSR) return false;
-  return c->has_q ? cluster_fits<QKernel>(c->device, resident_kernel<EpiQX, EpiQT, EpiY, EpiW2>, c->res.ctas)
-                  : cluster_fits<NoQKernel>(c->device, resident_kernel<EpiX, EpiY, EpiY, EpiY>, c->res.ctas);
+  return c->has_q ? cluster_fits(c->device, resident_kernel<EpiQX, EpiQT, EpiY, EpiW2>, c->res.ctas)
+                  : cluster_fits(c->device, resident_kernel<EpiX, EpiY, EpiY, EpiY>, c->res.ctas);
 }
 
 namespace {
+struct ResDotF {
+  const double* a;
+  __device__ void operator()(int64_t i, Red& r) const { r.v[0] = r.v[0] + a[i] * a[i]; }
+};
+
 // The matrices and tiles of the first `ns` sides.
 void resident_sides(const Ctx* c, int ns, ResArgs& a) {
   const Plan* plans[3] = {&c->planX, &c->planY, &c->planQ};
@@ -851,29 +841,45 @@ void resident_sides(const Ctx* c, int ns, ResArgs& a) {
 int launch_resident_power(Ctx* c, int maxit, double tol, double* lam, bool* done) {
   *done = false;
   if (c->res.ctas == 0 || c->m == 0) return HPR_OK;
+  const bool two = !(one_cta_plan(c->planX) && one_cta_plan(c->planY));
+  const int slots = c->planY.nslots();
+  if (two && slots > 2 * kThreads) return HPR_OK;  // its sums are two-level there
   HPR_TRY(prepare_engine(c));
   ResArgs a = ResArgs();
   int g[3] = {0, 0, 0};
-  // one more vector of length m (q) behind the batch's layout without Q
+  // q behind the batch's layout without Q
   const int64_t base = resident_layout(c, c->res, &a, g, false);
-  const int64_t smem = base + 8 * c->m;
-  if (smem > kResSmemMax || !cluster_fits(c->device, resident_power_kernel, c->res.ctas)) return HPR_OK;
+  const int64_t smem = base + (two ? 0 : 8 * c->m);
+  if (smem > kResSmemMax ||
+      !(two ? cluster_fits(c->device, resident_power_kernel<true>, c->res.ctas)
+            : cluster_fits(c->device, resident_power_kernel<false>, c->res.ctas)))
+    return HPR_OK;
   resident_sides(c, 2, a);
   a.st = c->d_state;
   std::vector<double> hz(c->m);
   power_start_vector(hz, 1);
   HPR_CUDA(c, cudaMemcpyAsync(c->pz, hz.data(), c->m * sizeof(double), cudaMemcpyHostToDevice, c->stream));
+  constexpr int kOut = 40;  // result lanes: lambda and iterations, then |z|^2, |z_new|^2, <z_old, z_new>
+  if (two) HPR_TRY(vec_reduce<1, 0>(c, c->m, ResDotF{c->pz}, kOut + 2));
+  const ResPower p{c->pz, c->pq, c->d_red_out + kOut + 2, c->d_red_out + kOut + 3, c->d_red_out + kOut,
+                   (int)c->m, maxit, slots, tol};
+  EpiScale es{};
+  es.out = c->ptq;
+  EpiPow ep{};
+  ep.lin_src[0] = ep.cone_src[0] = c->pz;
   const RStage<EpiPlain> sat{plain(c->ptq), 0, (int)base, g[1], c->ptq, 1, nullptr};
   const RStage<EpiPlain> sa{plain(c->pz), 1, g[1], g[0], c->pq, 1, nullptr};
+  const RStage<EpiScale> ss{es, 0, g[0], g[1], c->ptq, 1, nullptr};
+  const RStage<EpiPow> sp{ep, 1, g[1], g[0], c->pq, 1, c->d_red};
   cudaLaunchAttribute attr[1];
   const cudaLaunchConfig_t cfg = resident_config(c->res.ctas, smem, c->stream, attr);
-  HPR_CUDA(c, cudaLaunchKernelEx(&cfg, resident_power_kernel, a, sat, sa, (const double*)c->pz, (int)c->m, maxit, tol,
-                                 c->d_red_out + 40));
+  if (two) HPR_CUDA(c, cudaLaunchKernelEx(&cfg, resident_power_kernel<true>, a, sat, sa, ss, sp, p));
+  else HPR_CUDA(c, cudaLaunchKernelEx(&cfg, resident_power_kernel<false>, a, sat, sa, ss, sp, p));
   c->launches++;
-  HPR_CUDA(c, cudaMemcpyAsync(c->h_red_out + 40, c->d_red_out + 40, 2 * sizeof(double), cudaMemcpyDeviceToHost,
+  HPR_CUDA(c, cudaMemcpyAsync(c->h_red_out + kOut, c->d_red_out + kOut, 2 * sizeof(double), cudaMemcpyDeviceToHost,
                               c->stream));
   HPR_CUDA(c, cudaStreamSynchronize(c->stream));
-  *lam = c->h_red_out[40];
+  *lam = c->h_red_out[kOut];
   *done = true;
   return HPR_OK;
 }

@@ -40,8 +40,7 @@ def test_one_wave_of_wide_tiles_and_more(scale):
 
 
 # (rows of A about n / 2, 3.5% dense: one CTA, then clusters of 2 to 16 CTAs,
-# then past the largest; 48 to 56 and 1,100 have cones split over tiles or one
-# tile's 33rd row)
+# then past the largest; from about 1,100 cones are split over tiles)
 @pytest.mark.parametrize("n", [50, 56, 120, 400, 690, 803, 1100, 1700, 2300, 2900, 3600])
 @pytest.mark.parametrize("diag_q", [False, True])
 def test_cluster_resident_batches(n, diag_q):
