@@ -695,7 +695,7 @@ __global__ void bounds_box_kernel(int64_t n, const double* l, const double* u, c
 }
 // compute_err_soc_kernel! (kernels.jl:6617-6655).  A warp per cone, the lanes
 // striding over its rows (one thread per cone read a 5000-row cone alone: 2.34
-// ms of a re-solve at n = 2M and 0.6 ms at n = 100k, 20 us here); cones of up
+// ms of a re-solve at n = 2M and 0.6 ms at n = 100k); cones of up
 // to kSerialCone rows are taken 32 at a time, one per lane.
 constexpr int kSerialCone = 8;
 __device__ __forceinline__ void bounds_row(int64_t j, bool head, double t, double ns, const double* xb,
@@ -715,8 +715,10 @@ __global__ void bounds_cone_kernel(int64_t ncones, const int32_t* vs, const doub
   const int lane = threadIdx.x & 31;
   const int64_t w = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
-  for (int64_t k0 = 32 * w; k0 < ncones; k0 += 32 * nw) {
-    const int64_t k = k0 + lane;
+  // (lane l's cone is nw cones after lane l - 1's: neighbouring cones, which
+  // are often of one size, go to different warps)
+  for (int64_t k0 = w; k0 < ncones; k0 += 32 * nw) {
+    const int64_t k = k0 + nw * lane;
     const int32_t st = k < ncones ? vs[k] : 0, en = k < ncones ? vs[k + 1] : 0;
     const bool big = en - st > kSerialCone;
     if (!big && en > st) {
@@ -755,7 +757,7 @@ int launch_residuals(Ctx* c, bool include_bounds, hpr_residuals* r) {
     bounds_box_kernel<<<592, kThreads, 0, c->stream>>>(c->n, c->l, c->u, c->x_bar, c->col_norm, bs, c->dx);
     int64_t nv = (int64_t)c->h_var_idx.size() - 1;
     if (nv > 0)
-      bounds_cone_kernel<<<(int)std::min<int64_t>((nv + 127) / 128, 1184), 128, 0, c->stream>>>(
+      bounds_cone_kernel<<<(int)std::min<int64_t>((nv + 31) / 32, 1184), 128, 0, c->stream>>>(
           nv, c->d_var_start, c->x_bar, c->col_norm, bs, c->dx);
     HPR_CUDA(c, cudaGetLastError());
     HPR_TRY(vec_reduce<1, 1>(c, c->n, AbsMaxF{c->dx}, 16));
@@ -1547,7 +1549,7 @@ int launch_residuals_noalloc(Ctx* c, bool include_bounds, hpr_residuals* r) {
     bounds_box_kernel<<<592, kThreads, 0, c->stream>>>(c->n, c->l, c->u, c->x_bar, c->col_norm, bs, c->dx);
     int64_t nv = (int64_t)c->h_var_idx.size() - 1;
     if (nv > 0)
-      bounds_cone_kernel<<<(int)std::min<int64_t>((nv + 127) / 128, 1184), 128, 0, c->stream>>>(
+      bounds_cone_kernel<<<(int)std::min<int64_t>((nv + 31) / 32, 1184), 128, 0, c->stream>>>(
           nv, c->d_var_start, c->x_bar, c->col_norm, bs, c->dx);
     HPR_CUDA(c, cudaGetLastError());
     const int64_t len = c->n;

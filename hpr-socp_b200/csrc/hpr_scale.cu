@@ -134,6 +134,8 @@ __device__ __forceinline__ double group_combine(double v, bool sum) {
   return v;
 }
 
+constexpr int kLongRow = 96;  // entries past which a warp takes a row that a group of fewer lanes would walk
+
 // compute_row_max_abs(_with_Q)_kernel! / compute_row_sum_abs_kernel! /
 // compute_col_sum_abs_with_Q_kernel! (kernels.jl:6699-6798, 6965-7030)
 template <int G>
@@ -146,7 +148,25 @@ __global__ void row_stat_kernel(int64_t nr, const int32_t* rp, const double* v, 
   for (int64_t b0 = w * kRows; b0 < nr; b0 += nw * kRows) {
     const int64_t i = b0 + lane / G;
     double q = 0.0, a = 0.0;
-    if (i < nr) {
+    // one thread per row, maxima: a long row is left to the whole warp (a
+    // maximum does not depend on the order; measured on B200, A of the
+    // 500k-column SOCP with rows of up to 2000: 93 us per pass with one
+    // thread walking each)
+    const bool far = G == 1 && !use_sum && !qrp && i < nr && rp[i + 1] - rp[i] > kLongRow;
+    if constexpr (G == 1) {
+      unsigned todo = __ballot_sync(0xffffffffu, far);
+      while (todo) {
+        const int src = __ffs((int)todo) - 1;
+        todo &= todo - 1;
+        const int64_t r = b0 + src;
+        double x = 0.0;
+        for (int64_t k = rp[r] + lane; k < rp[r + 1]; k += 32) x = cmax(x, fabs(v[k]));
+        x = group_combine<32>(x, false);
+        x = __shfl_sync(0xffffffffu, x, 0);
+        if (lane == src) a = x;
+      }
+    }
+    if (i < nr && !far) {
       if (qrp)
         for (int64_t k = qrp[i] + sub; k < qrp[i + 1]; k += G) q = use_sum ? q + fabs(qv[k]) : cmax(q, fabs(qv[k]));
       for (int64_t k = rp[i] + sub; k < rp[i + 1]; k += G) a = use_sum ? a + fabs(v[k]) : cmax(a, fabs(v[k]));
@@ -193,6 +213,16 @@ __global__ void block_kernel(int64_t ncones, const int32_t* cs, double* t, int s
 }
 
 // scale_csr_row_col_kernel! (kernels.jl:7120-7140)
+__device__ __forceinline__ void scale_entries(double* v, const int32_t* ci, const double* cl, double rinv, int64_t b,
+                                              int64_t e, int step) {
+#pragma unroll 4
+  for (int64_t k = b; k < e; k += step) {
+    double x = v[k];
+    x *= rinv;
+    x /= cl[ci[k]];
+    v[k] = x;
+  }
+}
 template <int G>
 __global__ void scale_csr_kernel(int64_t nr, const int32_t* rp, const int32_t* ci, double* v, const double* r,
                                  const double* cl) {
@@ -202,13 +232,19 @@ __global__ void scale_csr_kernel(int64_t nr, const int32_t* rp, const int32_t* c
   const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
   for (int64_t b0 = w * kRows; b0 < nr; b0 += nw * kRows) {
     const int64_t i = b0 + lane / G;
-    if (i >= nr) continue;
-    const double rinv = 1.0 / r[i];
-    for (int64_t k = rp[i] + sub; k < rp[i + 1]; k += G) {
-      double x = v[k];
-      x *= rinv;
-      x /= cl[ci[k]];
-      v[k] = x;
+    const int64_t kb = i < nr ? rp[i] : 0, ke = i < nr ? rp[i + 1] : 0;
+    const bool far = G < 32 && ke - kb > kLongRow;
+    const double rinv = i < nr ? 1.0 / r[i] : 1.0;
+    if (!far) scale_entries(v, ci, cl, rinv, kb + sub, ke, G);
+    // a long row by the whole warp (223 us per pass for A of the 500k-column
+    // SOCP while groups of 8 lanes walked its rows of up to 2000 entries)
+    unsigned todo = __ballot_sync(0xffffffffu, far && sub == 0);
+    while (todo) {
+      const int src = __ffs((int)todo) - 1;
+      todo &= todo - 1;
+      const double ri = __shfl_sync(0xffffffffu, rinv, src);
+      const int64_t b = __shfl_sync(0xffffffffu, kb, src), e = __shfl_sync(0xffffffffu, ke, src);
+      scale_entries(v, ci, cl, ri, b + lane, e, 32);
     }
   }
 }
