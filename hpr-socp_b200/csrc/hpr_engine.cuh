@@ -8,12 +8,12 @@
 // nonzeros cut into 32 contiguous runs, lane-interleaved.
 //
 // Every warp works on its own tiles with no CTA-wide synchronisation, so the
-// SM's 24 resident warps hide each other's memory latency.  Persistent
+// SM's 24 resident warps (16 for small plans) hide each other's memory latency.  Persistent
 // warps take their first tile by warp index (plans without split cones) and
 // the rest from an atomic counter; per tile a warp
 //   1. streams its run's column indices and values with coalesced
-//      evict-first loads, gathers xin through L2 (ld.global.cg) and adds the
-//      products of each row inside the run in column order in a register,
+//      evict-first loads, gathers xin (through L1, or L2 only for a long
+//      vector: host-chosen) and adds the products of each row inside the run in column order in a register,
 //      closing a row's sum into a shared-memory slot at the next row start;
 //   2. adds the parts of rows that span runs with a fixed-order segmented
 //      scan over the lanes, and hands each row's sum to the lane that owns
@@ -118,7 +118,7 @@ __device__ void block_reduce(Red& r, double (*s_red)[kThreads / 32]) {
 }
 
 // Cache operators of the engine's loads (defaults measured best on B200:
-// gathers through L2 only, streams and epilogue inputs evict-first):
+// streams and epilogue inputs evict-first):
 //   col / val streams:   0 ld.global.cs, 1 ld.global.cg,
 //                        2 ld.global.nc.L1::no_allocate with an L2 evict-first
 //                          policy, 3 ld.global.nc;

@@ -367,12 +367,15 @@ int hpr_set_vector(hpr_ctx* ctx, int which, const double* host, size_t len);
 int hpr_get_solution(hpr_ctx* ctx, double* x, double* y, double* z, double* w);
 
 /* Iteration schedule (no counterpart in the reference, whose iteration is
- * always a sequence of separate kernels).  Problems whose matrix sides have
- * at most 32 warp tiles can run either on the multi-CTA engine (2 launches
- * per iteration, 4 with Q) or on one CTA that runs a whole batch of
- * iterations in a single launch.  AUTO (the default) times both on the
- * first batch of a size class in the process and keeps the faster; ENGINE
- * and FUSED force one.  The iterates are identical on every schedule.      */
+ * always a sequence of separate kernels).  AUTO (the default) runs a problem
+ * that fits the shared memory of one thread-block cluster (FP64, no Q or a CSR
+ * Q, no row longer than a tile) as one launch per batch of iterations.  Other
+ * problems whose matrix sides have at most 32 warp tiles run on the
+ * multi-CTA engine (2 launches per iteration, 4 with Q) or on one CTA that
+ * runs a whole batch in a single launch: AUTO times both on the first batch
+ * of a size class in the process and keeps the faster.  ENGINE forces the
+ * engine, FUSED a one-launch schedule where one applies.  The iterates are
+ * identical on every schedule.                                             */
 #define HPR_SCHEDULE_AUTO 0
 #define HPR_SCHEDULE_ENGINE 1
 #define HPR_SCHEDULE_FUSED 2
