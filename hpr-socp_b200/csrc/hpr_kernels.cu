@@ -324,12 +324,20 @@ int engine_launch(Ctx* c, const DevCSR& M, const Plan& p, const int32_t* cone_st
   a.st = c->d_state;
   a.red_slots = with_red ? c->d_red : nullptr;
   a.bump_inner = bump ? 1 : 0;
-  if (c->precision == HPR_PREC_FP32 && xin32 && M.val32)
-    launch_engine_prec<Epi, HPR_PREC_FP32>(c, nt, a, epi);
-  else if (c->precision == HPR_PREC_BF16 && xin32 && M.val16)
-    launch_engine_prec<Epi, HPR_PREC_BF16>(c, nt, a, epi);
-  else
-    launch_engine_prec<Epi, HPR_PREC_FP64>(c, nt, a, epi);
+  // (only the half-steps over A and A' pass an FP32 vector; the other
+  // epilogues' reduced-precision kernels would only lengthen the library's
+  // first load)
+  bool low = false;
+  if constexpr (std::is_same_v<Epi, EpiX> || std::is_same_v<Epi, EpiY>) {
+    low = true;
+    if (c->precision == HPR_PREC_FP32 && xin32 && M.val32)
+      launch_engine_prec<Epi, HPR_PREC_FP32>(c, nt, a, epi);
+    else if (c->precision == HPR_PREC_BF16 && xin32 && M.val16)
+      launch_engine_prec<Epi, HPR_PREC_BF16>(c, nt, a, epi);
+    else
+      low = false;
+  }
+  if (!low) launch_engine_prec<Epi, HPR_PREC_FP64>(c, nt, a, epi);
   c->launches++;
   HPR_CUDA(c, cudaGetLastError());
   if (with_red) {
