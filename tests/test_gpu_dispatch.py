@@ -98,3 +98,31 @@ def test_gathers_through_l1_and_past_it(scale):
     """1,040,000 and 1,060,000 columns: both sides of the line (2^20) below
     which the gathers go through L1."""
     _check(instances.config1(6, scale=scale), iters=3)
+
+
+@pytest.mark.parametrize("dims", [[2, 8, 3], [9, 8, 40, 3], [200, 7, 1500], [3] * 70 + [64, 65]])
+def test_bound_violation_by_lane_and_by_warp(dims):
+    """Cones of up to 8 rows (one lane) and above (a warp), more and fewer than
+    a warp's 32: the residuals with the bound violation at a start point that
+    is on both sides of every cone (norms regroup: 1e-12)."""
+    from hprsocp_b200 import Context, SOCPModel
+    import scipy.sparse as sp
+    rng = np.random.default_rng(len(dims))
+    nb, n, m = 6, 6 + sum(dims), 12
+    A = sp.random(m, n, density=0.3, random_state=rng, format="csr") + sp.eye(m, n, format="csr")
+    model = SOCPModel(A=A, c=rng.standard_normal(n), AL=-np.ones(m), AU=np.ones(m),
+                      l=np.r_[-np.ones(nb), np.full(n - nb, -np.inf)], u=np.r_[np.ones(nb), np.full(n - nb, np.inf)],
+                      soc_rhs=np.zeros(0), SOC_con_idx=np.array([m]),
+                      SOC_var_idx=np.concatenate([[nb], nb + np.cumsum(dims)]), number_linear_con=m, number_lu_x=nb)
+    with Context(model) as g:
+        o = OracleContext(model, threads=0)
+        p = HPRSOCP_parameters(verbose=False)
+        o.scale(p)
+        g.scale(p)
+        x = 3.0 * rng.standard_normal(n)
+        for c in (o, g):
+            c.set("x_bar", x)
+        a, b = g.residuals(True), o.residuals(True)
+        for k in b:
+            assert abs(a[k] - b[k]) <= 1e-12 * max(1.0, abs(b[k])), (k, a[k], b[k])
+        o.close()
