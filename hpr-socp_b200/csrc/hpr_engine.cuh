@@ -911,6 +911,12 @@ __global__ void __launch_bounds__(kThreads) final_reduce_kernel(const double* __
 // [b * per, (b + 1) * per) of slots in a fixed order (per from nslots and
 // the grid size only) into partial slot b.
 constexpr int kWideReduceCtas = 148;
+// chunks of the two-level reduction of `nslots` slots; 0: one level
+__host__ __device__ inline int wide_chunks(int nslots) {
+  if (nslots <= 2 * kThreads) return 0;
+  const int g = (nslots + kThreads - 1) / kThreads;
+  return g < kWideReduceCtas ? g : kWideReduceCtas;
+}
 template <int NRED, unsigned MASK>
 __global__ void __launch_bounds__(kThreads) slot_chunk_kernel(const double* __restrict__ slots, int nslots,
                                                               double* __restrict__ partial) {

@@ -342,12 +342,12 @@ int engine_launch(Ctx* c, const DevCSR& M, const Plan& p, const int32_t* cone_st
   HPR_CUDA(c, cudaGetLastError());
   if (with_red) {
     const int ns = p.nslots();
-    if (wide_reduce && ns > 2 * kThreads && c->d_red2) {
+    const int g = wide_reduce && c->d_red2 ? wide_chunks(ns) : 0;
+    if (g > 0) {
       // two fixed-order levels: contiguous chunks of slots per CTA, then
       // the chunk sums (one CTA reading tens of thousands of slots is a
       // tenth of a power-iteration step on the benchmark; 58 + 50 us of the
       // residual check's 390 there)
-      const int g = std::min<int>(kWideReduceCtas, (ns + kThreads - 1) / kThreads);
       slot_chunk_kernel<Epi::kNRed, Epi::kMaxMask><<<g, kThreads, 0, c->stream>>>(c->d_red, ns, c->d_red2);
       final_reduce_kernel<Epi::kNRed, Epi::kMaxMask><<<1, kThreads, 0, c->stream>>>(c->d_red2, g,
                                                                                      c->d_red_out + red_off);

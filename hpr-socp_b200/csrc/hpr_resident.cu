@@ -91,7 +91,8 @@ struct ResCheck {
   const double *x_bar, *y_bar;
   int n, m, on;
   int slots_x, slots_y;
-  double* out;  // Rd lanes at 0, Rp lanes at 8
+  double* partial;  // chunk sums of a two-level reduction
+  double* out;      // Rd lanes at 0, Rp lanes at 8
 };
 
 struct ResArgs {
@@ -478,14 +479,14 @@ __device__ __forceinline__ void res_stage(const RStage<E>& st, const ResArgs& a,
   res_sync(C);
 }
 
-// Slots in final_reduce_kernel's order (kThreads strides, then the block's
-// warps), by the first kThreads threads of one CTA; every thread calls it.
+// Slots b to e in final_reduce_kernel's order (kThreads strides, then the
+// block's warps), by the first kThreads threads of one CTA; every thread calls it.
 template <class E>
-__device__ void res_final(const double* slots, int nslots, double* out, double (*s_red)[kThreads / 32]) {
+__device__ void res_combine(const double* slots, int b, int e, double* out, double (*s_red)[kThreads / 32]) {
   Red r;
   red_init<E::kNRed, E::kMaxMask>(r);
   if (threadIdx.x < kThreads) {
-    for (int q = threadIdx.x; q < nslots; q += kThreads) {
+    for (int q = b + threadIdx.x; q < e; q += kThreads) {
       Red o;
 #pragma unroll
       for (int k = 0; k < E::kNRed; ++k) o.v[k] = __ldcg(slots + (int64_t)q * kMaxRed + k);
@@ -512,6 +513,22 @@ __device__ void res_final(const double* slots, int nslots, double* out, double (
   __syncthreads();
 }
 
+// All slots of a side, in one level or, where engine_launch takes two, in its
+// chunks: the host decides on residuals that must not depend on the schedule.
+template <class E>
+__device__ void res_final(const double* slots, int nslots, double* partial, double* out,
+                          double (*s_red)[kThreads / 32]) {
+  const int g = wide_chunks(nslots);
+  if (g > 0) {
+    const int per = (nslots + g - 1) / g;
+    for (int b = 0; b < g; ++b)
+      res_combine<E>(slots, b * per, min(b * per + per, nslots), partial + (int64_t)b * kMaxRed, s_red);
+    slots = partial;
+    nslots = g;
+  }
+  res_combine<E>(slots, 0, nslots, out, s_red);
+}
+
 // The residual lanes of the batch's last (full) iterate: x_bar and y_bar
 // replace the gathered copies, and the passes of launch_residuals run over
 // the tiles that are already in shared memory.  (As separate launches the
@@ -529,8 +546,8 @@ __device__ void res_check(const ResCheck& k, const ResArgs& a, unsigned char* sm
   res_stage(k.rd, a, sm, cur, false, ws, rank, C);
   res_stage(k.rp, a, sm, cur, false, ws, rank, C);
   if (rank == 0) {
-    res_final<EpiRd>(k.rd.slots, k.slots_x, k.out, s_red);
-    if (k.rp.on) res_final<EpiRp>(k.rp.slots, k.slots_y, k.out + 8, s_red);
+    res_final<EpiRd>(k.rd.slots, k.slots_x, k.partial, k.out, s_red);
+    if (k.rp.on) res_final<EpiRp>(k.rp.slots, k.slots_y, k.partial, k.out + 8, s_red);
   }
 }
 
@@ -633,7 +650,7 @@ __global__ void __launch_bounds__(kResThreads, 1)
       s2.e.lin_src[0] = (it & 1) ? p.z2 : p.z;
       s2.gglob = (it & 1) ? p.z : p.z2;
       res_stage(s2, a, sm, st, false, ws, rank, C);
-      if (rank == 0) res_final<EpiPow>(sp.slots, p.slots, p.lanes, s_red);
+      if (rank == 0) res_combine<EpiPow>(sp.slots, 0, p.slots, p.lanes, s_red);
       res_sync(C);
       const double nn2 = __ldcg(p.lanes), dot = __ldcg(p.lanes + 1);
       lambda = dot / sqrt(nz2);
@@ -843,7 +860,7 @@ int launch_resident_power(Ctx* c, int maxit, double tol, double* lam, bool* done
   if (c->res.ctas == 0 || c->m == 0) return HPR_OK;
   const bool two = !(one_cta_plan(c->planX) && one_cta_plan(c->planY));
   const int slots = c->planY.nslots();
-  if (two && slots > 2 * kThreads) return HPR_OK;  // its sums are two-level there
+  if (two && wide_chunks(slots) > 0) return HPR_OK;  // its sums are two-level there
   HPR_TRY(prepare_engine(c));
   ResArgs a = ResArgs();
   int g[3] = {0, 0, 0};
@@ -913,6 +930,7 @@ int launch_resident(Ctx* c, int64_t k, bool full_last, bool check) {
     chk.m = (int)c->m;
     chk.slots_x = c->planX.nslots();
     chk.slots_y = c->planY.nslots();
+    chk.partial = c->d_red2;
     chk.out = c->d_red_out + kCheckLanes;
   }
   cudaLaunchAttribute attr[1];

@@ -1,0 +1,46 @@
+"""The schedules (hpr_set_schedule) against one another: which kernels a
+problem gets, and that iterates, residuals and lambda are the same to the
+bit on all of them."""
+import numpy as np
+import pytest
+import scipy.sparse as sp
+
+from hprsocp_b200 import HPRSOCP_parameters, instances
+
+pytestmark = pytest.mark.gpu
+
+
+def _split_cones(seed, n, m, diag_q=False):
+    """n variables, nearly all in cones of 65 rows (two slices and two apply
+    tiles each), 3 nonzeros per row: more than 512 reduction slots on the
+    variables' side for n from about 8,000."""
+    rng = np.random.default_rng(seed)
+    kv, kc = int(0.9 * n) // 65, m // 15
+    A1 = instances._random_rows(rng, m - 5 * kc, n, np.full(m - 5 * kc, 3))
+    A2 = instances._random_rows(rng, 5 * kc, n, np.full(5 * kc, 3))
+    model = instances._assemble(rng, A1, A2, n - 65 * kv, [65] * kv, [5] * kc)
+    if diag_q:
+        model.Q = sp.diags(rng.uniform(0.0, 1.0, size=n)).tocsr()
+        model.__post_init__()
+    return model
+
+
+@pytest.mark.parametrize("iters", [20, 50, 140])
+def test_residuals_of_a_batch_past_512_slots(iters):
+    """Above 512 reduction slots the residual passes add in two levels; the
+    lanes that come with a cluster-resident batch add in the same order, so a
+    solve reports the same residuals on both schedules, to the bit."""
+    from hprsocp_b200 import Context
+    model = _split_cones(1, 10000, 3000)
+    res = {}
+    for mode in ("auto", "engine"):
+        with Context(model) as g:
+            g.set_schedule(mode)
+            r = g.solve(HPRSOCP_parameters(verbose=False, stoptol=1e-14, max_iter=iters))
+            assert r.iter == iters
+            assert r.last == g.residuals(), mode
+            res[mode] = r
+            g.iterate(4, True)
+            assert g.last_iterate()[1] == (1 if mode == "auto" else 8)
+    assert res["auto"].last == res["engine"].last
+    assert np.array_equal(res["auto"].x, res["engine"].x)
