@@ -1451,9 +1451,9 @@ double iteration_bytes(const Ctx* c) {
 // Allocation-free residual evaluation (hpr_compute_residuals_noalloc).
 //
 // Same kernels and reduction order as launch_residuals, but the per-tile
-// reduction slots, the per-block partials of the bound check and the result
-// lanes live in a file-scope device array instead of the context's
-// reduction buffers, and the read-back goes to the caller's stack instead of
+// reduction slots, their chunk sums, the per-block partials of the bound check
+// and the result lanes live in a file-scope device array instead of the
+// context's reduction buffers, and the read-back goes to the caller's stack instead of
 // the context's pinned buffer.  Nothing here starts at zero: every slot is
 // written by the tile (or finishing warp) that owns it before
 // final_reduce_kernel reads it, so the array needs no initialisation and
@@ -1463,10 +1463,11 @@ namespace {
 
 constexpr int64_t kNoAllocScratchBytes = (int64_t)2 << 20;  // 2 MiB
 constexpr int64_t kNoAllocDoubles = kNoAllocScratchBytes / (int64_t)sizeof(double);
-constexpr int64_t kNoAllocOut = 24;  // result lanes at the end of the array
+constexpr int64_t kNoAllocOut = 24;  // result lanes at the end of the 2 MiB
+constexpr int64_t kNoAllocChunks = (int64_t)kWideReduceCtas * kMaxRed;  // chunk sums, behind them
 constexpr int kNoAllocMaxDevices = 64;
 
-static __device__ __align__(256) double g_noalloc_scratch[kNoAllocDoubles];
+static __device__ __align__(256) double g_noalloc_scratch[kNoAllocDoubles + kNoAllocChunks];
 
 std::mutex g_noalloc_mu[kNoAllocMaxDevices];  // one call at a time per device
 double* g_noalloc_ptr[kNoAllocMaxDevices] = {};
@@ -1485,10 +1486,10 @@ int noalloc_scratch(Ctx* c, double** out) {
   return HPR_OK;
 }
 
-// engine_launch with caller-given reduction slots and result lanes.
+// engine_launch with caller-given reduction slots, chunk sums and result lanes.
 template <class Epi>
 int engine_launch_into(Ctx* c, const DevCSR& M, const Plan& p, const int32_t* cone_start, const double* xin,
-                       const Epi& epi, double* slots, double* out) {
+                       const Epi& epi, double* slots, double* chunks, double* out) {
   const int nt = (int)p.tasks.size();
   if (nt == 0) {
     HPR_CUDA(c, cudaMemsetAsync(out, 0, Epi::kNRed * sizeof(double), c->stream));
@@ -1508,7 +1509,15 @@ int engine_launch_into(Ctx* c, const DevCSR& M, const Plan& p, const int32_t* co
   launch_engine_prec<Epi, HPR_PREC_FP64>(c, nt, a, epi);
   c->launches++;
   HPR_CUDA(c, cudaGetLastError());
-  final_reduce_kernel<Epi::kNRed, Epi::kMaxMask><<<1, kThreads, 0, c->stream>>>(slots, p.nslots(), out);
+  int ns = p.nslots();
+  const int g = wide_chunks(ns);
+  if (g > 0) {
+    slot_chunk_kernel<Epi::kNRed, Epi::kMaxMask><<<g, kThreads, 0, c->stream>>>(slots, ns, chunks);
+    c->launches++;
+    slots = chunks;
+    ns = g;
+  }
+  final_reduce_kernel<Epi::kNRed, Epi::kMaxMask><<<1, kThreads, 0, c->stream>>>(slots, ns, out);
   c->launches++;
   HPR_CUDA(c, cudaGetLastError());
   return HPR_OK;
@@ -1532,6 +1541,7 @@ int launch_residuals_noalloc(Ctx* c, bool include_bounds, hpr_residuals* r) {
   double* scratch = nullptr;
   HPR_TRY(noalloc_scratch(c, &scratch));
   double* out = scratch + (kNoAllocDoubles - kNoAllocOut);
+  double* chunks = scratch + kNoAllocDoubles;
   const double bs = c->b_scale, cs = c->c_scale;
   const bool skipq = !c->has_q;
   // lanes of `out`: [0..5] Rd, [8..12] Rp, [16] bounds (as launch_residuals)
@@ -1541,7 +1551,7 @@ int launch_residuals_noalloc(Ctx* c, bool include_bounds, hpr_residuals* r) {
   for (int k = 0; k < 5; ++k) ed.lin_src[k] = ed.cone_src[k] = dsrc[k];
   ed.hasq = skipq ? 0 : 1;
   ed.cs = cs;
-  HPR_TRY(engine_launch_into(c, c->AT, c->planX, c->d_var_start, c->y_bar, ed, scratch, out));
+  HPR_TRY(engine_launch_into(c, c->AT, c->planX, c->d_var_start, c->y_bar, ed, scratch, chunks, out));
   if (c->m > 0) {
     EpiRp ep{};
     const double* psrc[5] = {c->AL, c->AU, c->row_norm, c->y_bar, c->s};
@@ -1551,7 +1561,7 @@ int launch_residuals_noalloc(Ctx* c, bool include_bounds, hpr_residuals* r) {
       ep.cone_src[k] = pcone[k];
     }
     ep.bs = bs;
-    HPR_TRY(engine_launch_into(c, c->A, c->planY, c->d_con_start, c->x_bar, ep, scratch, out + 8));
+    HPR_TRY(engine_launch_into(c, c->A, c->planY, c->d_con_start, c->x_bar, ep, scratch, chunks, out + 8));
   }
   if (include_bounds) {
     bounds_box_kernel<<<592, kThreads, 0, c->stream>>>(c->n, c->l, c->u, c->x_bar, c->col_norm, bs, c->dx);

@@ -310,9 +310,10 @@ int hpr_compute_residuals(hpr_ctx* ctx, int include_bounds,
  * (cudaMalloc may block; cudaFree and cudaFreeHost synchronise the whole
  * device and so stall every other stream).  This call allocates nothing: no
  * device, pinned or pageable allocation, no library routine that allocates.
- * Its reduction slots and result lanes live in a statically reserved 2 MiB
- * device array (reserved once per process and device when the library's
- * CUDA module loads), and its results go through the caller's stack.
+ * Its reduction slots and result lanes live in a statically reserved device
+ * array (2 MiB for them and 9 KiB for chunk sums, reserved once per process
+ * and device when the library's CUDA module loads), and its results go
+ * through the caller's stack.
  *
  * Limits and rules:
  *  - the problem's tile plan must fit the 2 MiB: at most 32,765 reduction

@@ -44,3 +44,14 @@ def test_residuals_of_a_batch_past_512_slots(iters):
             assert g.last_iterate()[1] == (1 if mode == "auto" else 8)
     assert res["auto"].last == res["engine"].last
     assert np.array_equal(res["auto"].x, res["engine"].x)
+
+
+@pytest.mark.parametrize("iters", [20, 50, 140])
+def test_allocation_free_residuals_past_512_slots(iters):
+    """hpr_compute_residuals_noalloc adds its slots as hpr_compute_residuals
+    does, also where that takes two levels."""
+    from hprsocp_b200 import Context
+    with Context(_split_cones(1, 10000, 3000)) as g:
+        g.solve(HPRSOCP_parameters(verbose=False, stoptol=1e-14, max_iter=iters))
+        for bounds in (False, True):
+            assert g.residuals_noalloc(bounds) == g.residuals(bounds)
