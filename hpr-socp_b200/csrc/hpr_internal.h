@@ -318,12 +318,12 @@ int launch_iteration(Ctx* c, bool full);
 // check: the caller wants the residuals of the last iterate next; *checked is
 // true when their lanes were computed with the batch (finish_residuals)
 int run_iterations(Ctx* c, int64_t k, bool full_last, bool check = false, bool* checked = nullptr);
-// true when run_iterations may use the single-CTA multi-iteration kernel
-// (then no partial-iteration graph is captured)
+// true when run_iterations may run whole batches in one launch, on a cluster or
+// on a single CTA (then no partial-iteration graph is captured)
 bool uses_fused_iterations(const Ctx* c);
 // cluster-resident batches (hpr_resident.cu)
 void resident_plan(Ctx* c);  // after the plans are built, before upload_plan
-bool resident_eligible(const Ctx* c);
+bool resident_eligible(const Ctx* c);  // on the automatic schedule only
 int launch_resident(Ctx* c, int64_t k, bool full_last, bool check);
 int launch_residuals(Ctx* c, bool include_bounds, hpr_residuals* out);
 // reads the residual lanes back (Rd's from lane `base` of d_red_out, Rp's from

@@ -649,7 +649,7 @@ int tune_trial(Ctx* c, int64_t k, bool full_last) {
 }  // namespace
 
 bool uses_fused_iterations(const Ctx* c) {
-  if (c->schedule != HPR_SCHEDULE_ENGINE && resident_eligible(c)) return true;
+  if (resident_eligible(c)) return true;
   if (!fused_eligible(c)) return false;
   const int mode = c->schedule != HPR_SCHEDULE_AUTO ? c->schedule : tune_lookup(c);
   return mode != HPR_SCHEDULE_ENGINE;
@@ -661,7 +661,7 @@ int run_iterations(Ctx* c, int64_t k, bool full_last, bool check, bool* checked)
   int64_t l0 = c->launches;
   HPR_CUDA(c, cudaEventRecord(c->ev0, c->stream));
   int mode = HPR_SCHEDULE_ENGINE;
-  if (c->schedule != HPR_SCHEDULE_ENGINE && resident_eligible(c)) {
+  if (resident_eligible(c)) {
     HPR_TRY(launch_resident(c, k, full_last, check && full_last));
     if (checked) *checked = check && full_last;
     HPR_CUDA(c, cudaEventRecord(c->ev1, c->stream));

@@ -819,7 +819,7 @@ void resident_plan(Ctx* c) {
 }
 
 bool resident_eligible(const Ctx* c) {
-  if (c->res.ctas == 0 || c->precision != HPR_PREC_FP64) return false;
+  if (c->schedule != HPR_SCHEDULE_AUTO || c->res.ctas == 0 || c->precision != HPR_PREC_FP64) return false;
   if (c->q_kind != HPR_Q_NONE && c->q_kind != HPR_Q_CSR) return false;
   return c->has_q ? cluster_fits(c->device, resident_kernel<EpiQX, EpiQT, EpiY, EpiW2>, c->res.ctas)
                   : cluster_fits(c->device, resident_kernel<EpiX, EpiY, EpiY, EpiY>, c->res.ctas);
@@ -857,7 +857,7 @@ void resident_sides(const Ctx* c, int ns, ResArgs& a) {
 
 int launch_resident_power(Ctx* c, int maxit, double tol, double* lam, bool* done) {
   *done = false;
-  if (c->res.ctas == 0 || c->m == 0) return HPR_OK;
+  if (c->schedule != HPR_SCHEDULE_AUTO || c->res.ctas == 0 || c->m == 0) return HPR_OK;
   const bool two = !(one_cta_plan(c->planX) && one_cta_plan(c->planY));
   const int slots = c->planY.nslots();
   if (two && wide_chunks(slots) > 0) return HPR_OK;  // its sums are two-level there

@@ -276,7 +276,8 @@ class Context:
         return x, y, z, w
 
     def set_schedule(self, mode: str):
-        """'auto' (timed choice per size class), 'engine' or 'fused'."""
+        """'auto' (a cluster's shared memory where the problem fits it, else a
+        timed choice per size class), 'engine' or 'fused' (one CTA)."""
         self._check(self.lib.hpr_set_schedule(self.h, _abi.HPR_SCHEDULE[mode]))
 
     def set_precision(self, mode: str):

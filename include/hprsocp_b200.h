@@ -375,8 +375,9 @@ int hpr_get_solution(hpr_ctx* ctx, double* x, double* y, double* z, double* w);
  * multi-CTA engine (2 launches per iteration, 4 with Q) or on one CTA that
  * runs a whole batch in a single launch: AUTO times both on the first batch
  * of a size class in the process and keeps the faster.  ENGINE forces the
- * engine, FUSED a one-launch schedule where one applies.  The iterates are
- * identical on every schedule.                                             */
+ * engine; FUSED forces the single CTA for problems of at most 32 tiles per
+ * side (others run on the engine).  Iterates, residuals and the eigenvalue
+ * estimate are identical on every schedule.                                */
 #define HPR_SCHEDULE_AUTO 0
 #define HPR_SCHEDULE_ENGINE 1
 #define HPR_SCHEDULE_FUSED 2

@@ -55,3 +55,25 @@ def test_allocation_free_residuals_past_512_slots(iters):
         g.solve(HPRSOCP_parameters(verbose=False, stoptol=1e-14, max_iter=iters))
         for bounds in (False, True):
             assert g.residuals_noalloc(bounds) == g.residuals(bounds)
+
+
+@pytest.mark.parametrize("n,launches", [(60, {"auto": 1, "fused": 1, "engine": 24}),
+                                        (2000, {"auto": 1, "fused": 24, "engine": 24})])
+def test_each_schedule_runs_its_kernels(n, launches):
+    """A problem of a few tiles runs on one CTA when that is asked for; one of
+    more than 32 tiles per side then runs on the engine.  The cluster's
+    shared memory is the automatic schedule's.  lambda_max(AA') comes from a
+    different kernel on each and has the same bits."""
+    from hprsocp_b200 import Context
+    model = instances.small_socp(5 + n, n=n, diag_q=False)
+    lam = {}
+    for mode, count in launches.items():
+        with Context(model) as g:
+            g.set_schedule(mode)
+            info = g.scale(HPRSOCP_parameters(verbose=False))
+            lam[mode] = g.power_A()
+            g.set_sigma_lambda(info["norm_b"] / info["norm_c"], 1.05 * lam[mode], 0.0)
+            g.set_inner(0)
+            g.iterate(12, True)
+            assert g.last_iterate()[1] == count, mode
+    assert lam["auto"] == lam["fused"] == lam["engine"]
