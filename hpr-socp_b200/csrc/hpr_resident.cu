@@ -784,11 +784,16 @@ bool cluster_fits(int device, K kernel, int C) {
 // The cluster size for the context's problem and the slot offsets of its plans'
 // tiles in their CTA's shared memory (TileRun.soff).  c->res.ctas is 0 when the
 // problem does not fit the largest cluster or a side has a row longer than a
-// tile.  The smallest cluster that holds it is taken: a larger one only adds
-// barriers to the same chains (measured on B200, us per iteration on 1 / 2 / 4 /
-// 8 / 16 CTAs with an earlier form of the sums: n = 61 4.3 / 5.3 / 5.1 / 5.2 /
-// 5.1, n = 400 9.9 / 10.5 / 10.2 / 10.3 / 10.9), and the other SMs serve other
-// contexts.
+// tile.  The smallest cluster is taken that holds it with at most one tile per
+// warp (or 16 CTAs).  More CTAs only add barriers to the same chains, and the
+// other SMs serve other contexts (measured on B200, us per iteration on 1 / 2 /
+// 4 / 8 / 16 CTAs: n = 61 5.3 / 6.3 / 6.2 / 6.3 / 6.7, n = 400 7.6 / 8.3 / 8.6 /
+// 8.8 / 9.3).  With fewer than one warp per tile a warp works on
+// one tile after another, and a problem of few nonzeros per row has many tiles
+// in little memory (ms per 150-iteration solve in the smallest cluster that
+// holds it / with this rule / on separate launches: n = 3000, 2 nonzeros per row,
+// cones of 33 3.77 / 2.00 / 2.77; n = 6000, cones of 3 3.06 / 1.98 / 2.85; n =
+// 3000, diagonal Q, cones of 33 5.97 / 3.92 / 5.10).
 void resident_plan(Ctx* c) {
   c->res = ResidentShape();
   ResidentShape r;
@@ -798,7 +803,11 @@ void resident_plan(Ctx* c) {
   for (int i = 0; i < ns; ++i)
     if (!plans[i]->lng.empty()) return;
   if (plans[0]->tasks.empty() || (c->A.nnz + c->Q.nnz) / kResMaxCtas * 20 > kResSmemMax) return;
-  for (r.ctas = 1; r.ctas <= kResMaxCtas; r.ctas *= 2) {
+  int most = 0;  // tiles of the largest side
+  for (int i = 0; i < ns; ++i) most = std::max(most, nwork_of(*plans[i]));
+  r.ctas = 1;
+  while (r.ctas < kResMaxCtas && most > kResWarps * r.ctas) r.ctas *= 2;
+  for (; r.ctas <= kResMaxCtas; r.ctas *= 2) {
     const int C = r.ctas;
     for (int i = 0; i < ns; ++i) {
       Plan& p = *plans[i];

@@ -77,3 +77,33 @@ def test_each_schedule_runs_its_kernels(n, launches):
             g.iterate(12, True)
             assert g.last_iterate()[1] == count, mode
     assert lam["auto"] == lam["fused"] == lam["engine"]
+
+
+@pytest.mark.parametrize("n,dim,diag_q", [(3000, 33, False), (6000, 3, False), (1500, 33, True)])
+def test_a_sparse_small_problem_is_not_slower_on_the_automatic_schedule(n, dim, diag_q):
+    """Two nonzeros per row: many tiles in little memory.  A cluster just large
+    enough to hold them left each warp several tiles in a row and took 1.2 to
+    1.6 times the engine's iteration; with one tile per warp it takes 0.6 to
+    0.75 times (best of 9 batches each, in turn)."""
+    from hprsocp_b200 import Context
+    rng = np.random.default_rng(n + dim)
+    kv, kc = n // 2 // dim, n // 6 // dim
+    m2 = dim * kc
+    rows = [instances._random_rows(rng, r, n, np.full(r, 2)) for r in (n // 2 - m2, m2)]
+    model = instances._assemble(rng, *rows, n - dim * kv, [dim] * kv, [dim] * kc)
+    if diag_q:
+        model.Q = sp.diags(rng.uniform(0.0, 1.0, size=n)).tocsr()
+        model.__post_init__()
+    best = {"auto": np.inf, "engine": np.inf}
+    with Context(model) as g:
+        info = g.scale(HPRSOCP_parameters(verbose=False))
+        g.set_sigma_lambda(info["norm_b"] / info["norm_c"], 1.05 * g.power_A(), 0.0)
+        g.set_inner(0)
+        for _ in range(9):
+            for mode in best:
+                g.set_schedule(mode)
+                g.iterate(150, True)
+                ms, launches = g.last_iterate()
+                assert (launches == 1) == (mode == "auto")
+                best[mode] = min(best[mode], ms)
+    assert best["auto"] <= best["engine"], best
