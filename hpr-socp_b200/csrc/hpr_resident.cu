@@ -802,7 +802,8 @@ void resident_plan(Ctx* c) {
   const int ns = c->has_q ? 3 : 2;
   for (int i = 0; i < ns; ++i)
     if (!plans[i]->lng.empty()) return;
-  if (plans[0]->tasks.empty() || (c->A.nnz + c->Q.nnz) / kResMaxCtas * 20 > kResSmemMax) return;
+  // 10 bytes per nonzero; A is kept by rows and by columns (early out)
+  if (plans[0]->tasks.empty() || (20 * c->A.nnz + 10 * c->Q.nnz) / kResMaxCtas > kResSmemMax) return;
   int most = 0;  // tiles of the largest side
   for (int i = 0; i < ns; ++i) most = std::max(most, nwork_of(*plans[i]));
   r.ctas = 1;

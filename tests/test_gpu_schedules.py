@@ -107,3 +107,41 @@ def test_a_sparse_small_problem_is_not_slower_on_the_automatic_schedule(n, dim, 
                 assert (launches == 1) == (mode == "auto")
                 best[mode] = min(best[mode], ms)
     assert best["auto"] <= best["engine"], best
+
+
+def _general_q(seed, n, per_col, row_nnz):
+    """Q = B'B + D with B of `per_col` nonzeros per column in n/4 rows (about
+    4 n per_col^2 nonzeros of Q), A of n/2 rows of `row_nnz` nonzeros, cones of
+    20 and 25."""
+    rng = np.random.default_rng(seed)
+    kv, kc = n // 40, n // 150
+    rows = [instances._random_rows(rng, r, n, np.full(r, row_nnz)) for r in (n // 2 - 25 * kc, 25 * kc)]
+    model = instances._assemble(rng, *rows, n - 20 * kv, [20] * kv, [25] * kc)
+    B = sp.csr_matrix((rng.standard_normal(per_col * n),
+                       (rng.integers(0, n // 4, size=per_col * n), np.repeat(np.arange(n), per_col))),
+                      shape=(n // 4, n))
+    model.Q = (B.T @ B + sp.diags(rng.uniform(0.01, 1.0, size=n))).tocsr()
+    model.c = model.c - model.Q @ model.planted["x0"]
+    model.__post_init__()
+    return model
+
+
+@pytest.mark.parametrize("n,per_col,row_nnz,launches", [(2000, 5, 5, 1), (1500, 6, 10, 1), (4000, 4, 2, 48)])
+def test_a_problem_of_mostly_q_that_fits_the_cluster(n, per_col, row_nnz, launches):
+    """Q is kept once in the cluster's shared memory, A twice: 197,000 and
+    208,000 nonzeros of Q fit 16 CTAs beside 5,000 and 7,500 of A; 259,000 and
+    three copies of the vectors of n = 4000 do not."""
+    from hprsocp_b200 import Context
+    model = _general_q(n, n, per_col, row_nnz)
+    res = {}
+    for mode in ("auto", "engine"):
+        with Context(model) as g:
+            g.set_schedule(mode)
+            info = g.scale(HPRSOCP_parameters(verbose=False))
+            g.set_sigma_lambda(info["norm_b"] / info["norm_c"], 1.05 * g.power_A(), 1.05 * g.power_Q())
+            g.set_inner(0)
+            g.iterate(12, True)
+            assert g.last_iterate()[1] == (launches if mode == "auto" else 48)
+            res[mode] = [g.get(v) for v in ("x", "x_bar", "z_bar", "y", "y_bar", "s", "w", "w_bar", "ATy", "dx", "dy")]
+    for a, b in zip(res["auto"], res["engine"]):
+        assert np.array_equal(a, b)
