@@ -145,3 +145,87 @@ def test_a_problem_of_mostly_q_that_fits_the_cluster(n, per_col, row_nnz, launch
             res[mode] = [g.get(v) for v in ("x", "x_bar", "z_bar", "y", "y_bar", "s", "w", "w_bar", "ATy", "dx", "dy")]
     for a, b in zip(res["auto"], res["engine"]):
         assert np.array_equal(a, b)
+
+
+VECS = ["x", "x_hat", "x_bar", "z_bar", "y", "y_bar", "s", "dx", "dy"]
+QVECS = VECS + ["w", "w_bar", "ATy", "dw"]
+
+
+def _run(model, mode, batches=((70, True), (1, False), (30, True))):
+    """Iterates after the batches, the launches of each, lambda and the
+    residuals on one schedule."""
+    from hprsocp_b200 import Context
+    with Context(model) as g:
+        g.set_schedule(mode)
+        info = g.scale(HPRSOCP_parameters(verbose=False))
+        lam = g.power_A()
+        diag = model.Q is not None and (model.Q - sp.diags(model.Q.diagonal())).nnz == 0
+        lamq = 0.0 if model.Q is None or diag else 1.05 * g.power_Q()
+        g.set_sigma_lambda(info["norm_b"] / info["norm_c"], 1.05 * lam, lamq)
+        g.set_inner(0)
+        launches = []
+        for k, full in batches:
+            g.iterate(k, full)
+            launches.append(g.last_iterate()[1])
+        return ([g.get(v) for v in (VECS if model.Q is None else QVECS)] + [np.array(g.scalars()), np.array(lam)],
+                launches, g.residuals())
+
+
+def _same(a, b):
+    assert a[2] == b[2]
+    for u, v in zip(a[0], b[0]):
+        assert np.array_equal(u, v)
+
+
+# (with a diagonal Q one CTA up to n of about 400, then clusters of 2 to 16; a
+# general Q on 1 to 16; cones of 65 and more are split over tiles, which adds a
+# barrier in the half-steps that project)
+@pytest.mark.parametrize("kind,n", [("diag", 60), ("diag", 400), ("diag", 803), ("diag", 1200), ("diag", 2000),
+                                    ("general", 60), ("general", 300), ("general", 1000), ("general", 2500),
+                                    ("split", 1000), ("split", 2500), ("split_diag", 1000), ("split_diag", 2500),
+                                    ("split_diag", 5200)])
+def test_cluster_batches_are_the_engines_to_the_bit(kind, n):
+    """One launch per batch on the cluster, 2 or 4 per iteration on the engine;
+    iterates, lambda and residuals the same."""
+    if kind == "diag":
+        model = instances.small_socp(7 + n, n=n, diag_q=True)
+    elif kind == "general":
+        model = instances.qp_csr(n, n=n)
+    else:
+        model = _split_cones(n, n, n // 2, kind == "split_diag")
+    a, e = _run(model, "auto"), _run(model, "engine")
+    assert a[1] == [1, 1, 1]
+    per = 2 if model.Q is None else 4
+    assert e[1] == [70 * per, per, 30 * per]
+    _same(a, e)
+
+
+@pytest.mark.parametrize("n", [1100, 1600])
+@pytest.mark.parametrize("q", ["none", "general", "dense_row"])
+def test_single_cta_with_a_row_longer_than_a_tile(n, q):
+    """A dense budget row (and, in the last form, a dense row and column of Q)
+    of more than 1024 nonzeros keeps a problem of a few tiles out of the
+    cluster: it runs on one CTA, on the engine, or, at first, half on each to
+    choose.  All the same to the bit, and lambda too."""
+    rng = np.random.default_rng(n)
+    m1, kc, kv = 40, 8, n // 40
+    A1 = sp.vstack([sp.csr_matrix(rng.uniform(0.5, 1.5, size=(1, n))),
+                    instances._random_rows(rng, m1 - 1, n, np.full(m1 - 1, 5))]).tocsr()
+    A2 = instances._random_rows(rng, 5 * kc, n, np.full(5 * kc, 4))
+    model = instances._assemble(rng, A1, A2, n - 20 * kv, [20] * kv, [5] * kc)
+    if q == "general":
+        B = sp.random(20, n, density=12 / n, random_state=rng, data_rvs=rng.standard_normal, format="csr")
+        model.Q = (B.T @ B + sp.diags(rng.uniform(0.5, 1.0, size=n))).tocsr()
+    elif q == "dense_row":
+        arrow = sp.csr_matrix((np.full(n, 0.01), (np.full(n, 3), np.arange(n))), shape=(n, n))
+        model.Q = (arrow + arrow.T + sp.diags(rng.uniform(1.0, 2.0, size=n))).tocsr()
+    if q != "none":
+        model.c = model.c - model.Q @ model.planted["x0"]
+        model.__post_init__()
+    f, e, a = (_run(model, mode) for mode in ("fused", "engine", "auto"))
+    per = 2 if model.Q is None else 4
+    assert f[1] == [1, 1, 1]
+    assert e[1] == [70 * per, per, 30 * per]
+    assert a[1][0] in (1, 70 * per, 1 + 35 * per)  # already chosen in this process, or half on each
+    _same(f, e)
+    _same(a, e)
