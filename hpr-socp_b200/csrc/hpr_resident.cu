@@ -82,6 +82,10 @@ struct RStage {
   double* slots;  // reduction slots of the side's tiles (epilogues with reductions)
 };
 
+struct NoStage {};  // a half-step that the problem does not have
+template <>
+struct RStage<NoStage> {};
+
 // The residual check after a batch (compute_residuals!): the half-steps of
 // launch_residuals and where their lanes go.
 struct ResCheck {
@@ -450,6 +454,8 @@ __device__ __forceinline__ void res_apply(const ResSide& s, E& epi, int t, doubl
   if (gglob) publish_rows(gout, gglob, tk.rb, nrows, rank, C);
 }
 
+__device__ __forceinline__ void res_stage(const RStage<NoStage>&, const ResArgs&, unsigned char*, const DevState*,
+                                          bool, ResWs&, uint32_t, uint32_t) {}
 template <class E>
 __device__ __forceinline__ void res_stage(const RStage<E>& st, const ResArgs& a, unsigned char* sm,
                                           const DevState* cur, bool last, ResWs& ws, uint32_t rank, uint32_t C) {
@@ -832,7 +838,7 @@ bool resident_eligible(const Ctx* c) {
   if (c->schedule != HPR_SCHEDULE_AUTO || c->res.ctas == 0 || c->precision != HPR_PREC_FP64) return false;
   if (c->q_kind != HPR_Q_NONE && c->q_kind != HPR_Q_CSR) return false;
   return c->has_q ? cluster_fits(c->device, resident_kernel<EpiQX, EpiQT, EpiY, EpiW2>, c->res.ctas)
-                  : cluster_fits(c->device, resident_kernel<EpiX, EpiY, EpiY, EpiY>, c->res.ctas);
+                  : cluster_fits(c->device, resident_kernel<EpiX, EpiY, NoStage, NoStage>, c->res.ctas);
 }
 
 namespace {
@@ -952,8 +958,8 @@ int launch_resident(Ctx* c, int64_t k, bool full_last, bool check) {
     if (!c->has_q) {
       const RStage<EpiX> sx{E.ex, 0, g[0], g[1], c->x_hat, 1, nullptr};
       const RStage<EpiY> sy{E.ey, 1, g[1], g[0], c->y, hy, nullptr};
-      const RStage<EpiY> off{E.ey, 1, g[1], g[0], c->y, 0, nullptr};
-      HPR_CUDA(c, cudaLaunchKernelEx(&cfg, resident_kernel<EpiX, EpiY, EpiY, EpiY>, a, sx, sy, off, off, chk));
+      const RStage<NoStage> off;
+      HPR_CUDA(c, cudaLaunchKernelEx(&cfg, resident_kernel<EpiX, EpiY, NoStage, NoStage>, a, sx, sy, off, off, chk));
     } else {
       const RStage<EpiQX> sq{E.eq, 2, g[1], g[2], c->w_bar, 1, nullptr};
       const RStage<EpiQT> st{E.et, 2, g[2], g[1], c->tempv, hy, nullptr};
