@@ -214,8 +214,9 @@ struct EpiQX {
     finish(i, in, in(0, i), xb, zr);
   }
 };
-// (the Q path's x-step holds more state per row: two nonzeros per lane per
-// round keep it from spilling)
+// (the Q path's x-step holds more state per row than 80 registers: at two
+// nonzeros per lane per round it spills 32 to 40 bytes; the kWide form has the
+// registers for eight and spills nothing)
 template <int PREC>
 struct EngineChunk<EpiQX, PREC> {
   static constexpr int value = kChunk < 2 ? kChunk : 2;

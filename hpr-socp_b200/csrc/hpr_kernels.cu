@@ -266,7 +266,11 @@ void launch_engine_form(Ctx* c, int nt, const EngineArgs& a, const Epi& epi) {
 // are found there.  Measured on B200, us per iteration with L2-only gathers /
 // through L1: the Q path at n = 200k 136.1 / 102.8; uniformly random columns,
 // which find nothing, 55.4 / 55.4 at n = 300k, 97.7 / 98.0 at 700k, 153.0 /
-// 154.1 at 1.2M, 246.0 / 248.4 at 2M.
+// 154.1 at 1.2M, 246.0 / 248.4 at 2M.  (The gain depends on how near the columns
+// are and the line on the vector's length only: a longer vector with nearby
+// columns keeps the L2 form.)  The kWide form always goes through L1: random
+// columns of a few long rows cost it nothing (1000 rows of 1000 over n = 2M 60.1
+// / 60.1, 2000 over 4M 111.5 / 111.5, 20,000 rows of 60 over 2M 53.2 / 53.2).
 #ifndef HPR_GATHER_L1_MAX
 #define HPR_GATHER_L1_MAX (1 << 20)
 #endif

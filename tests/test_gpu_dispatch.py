@@ -126,3 +126,14 @@ def test_bound_violation_by_lane_and_by_warp(dims):
         for k in b:
             assert abs(a[k] - b[k]) <= 1e-12 * max(1.0, abs(b[k])), (k, a[k], b[k])
         o.close()
+
+
+def test_wide_tiles_over_more_columns_than_the_l1_line():
+    """600 rows of 300 nonzeros over 1,100,000 columns: the rows' side is one
+    wave of wide tiles, whose gathers go through L1 at any length, the columns'
+    side is past it."""
+    rng = np.random.default_rng(11)
+    n, kv = 1_100_000, 200
+    A1 = instances._random_rows(rng, 500, n, np.full(500, 300))
+    A2 = instances._random_rows(rng, 100, n, np.full(100, 300))
+    _check(instances._assemble(rng, A1, A2, n - 70 * kv, [70] * kv, [5] * 20), iters=3)
