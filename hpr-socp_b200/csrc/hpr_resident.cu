@@ -3,12 +3,12 @@
 //
 // A small problem's half-step is a chain of dependent memory round trips (tile
 // record, columns, gathers, epilogue inputs, stores) and of instructions, not
-// bytes.  Measured on B200, us per iteration of a 150-iteration batch, before
-// (single-CTA kernel through L2 up to n = 400, else the multi-CTA engine) and
-// here: n = 61 5.7 / 4.1, n = 400 12.0 / 7.4, n = 800 22 / 12.2, the same with
-// a diagonal Q 25.6 / 15.3, n = 2000 27.6 / 13.6, n = 3000 with a general CSR
-// Q 30 / 16.2.  What is left is the instruction chain of a tile: row sums,
-// cone norms, projections.
+// bytes.  Measured on B200, us per iteration of a 150-iteration batch on the
+// faster of the other schedules (single-CTA kernel through L2 up to n = 401,
+// else the multi-CTA engine) and here: n = 61 5.3 / 3.2, n = 401 10.0 / 5.7, n =
+// 803 18.2 / 10.5, with a diagonal Q 23.8 / 15.4, n = 2000 25.6 / 11.7, n = 3000
+// with a general CSR Q 26.3 / 16.0.  What is left is the instruction chain of a
+// tile: row sums, cone norms, projections.
 // Here every CTA of one cluster copies its share of the matrices (columns as
 // 16 bits, values in FP64, in the engine's run layout) and the tile records
 // into shared memory once per batch and keeps a full copy of each gathered
@@ -273,10 +273,10 @@ __device__ __forceinline__ void publish_rows(double* gout, double* gglob, int rb
 }
 
 // Row sums of a tile (process_warp_tile's steps 1 to 3).  The loads are not
-// conditional (padding is value 0, column 0, and its product is not used): a
-// branch around each load made every nonzero wait for the one before it (n =
-// 400: 9.9 us per iteration against 8.3), and generic pointers cost more
-// instructions than 32-bit shared addresses (8.3 against 7.2).
+// conditional (padding is value 0, column 0, and its product is not used) and
+// go through 32-bit shared addresses (us per iteration with a branch around each
+// load / through generic pointers / as here: n = 401 5.8 / 6.0 / 5.7, n = 2000
+// 11.9 / 12.2 / 11.5).
 __device__ __forceinline__ void run_sums(uint32_t val, uint32_t col, uint32_t xs, int nnz, uint64_t desc,
                                          uint64_t nonempty, uint32_t acc, double& acc0, double& acc1) {
   const int lane = threadIdx.x & 31;
@@ -537,9 +537,9 @@ __device__ void res_final(const double* slots, int nslots, double* partial, doub
 
 // The residual lanes of the batch's last (full) iterate: x_bar and y_bar
 // replace the gathered copies, and the passes of launch_residuals run over
-// the tiles that are already in shared memory.  (As separate launches the
-// check cost the host loop 50-65 us after every batch, a third of a solve at
-// n = 400: 16 checks in 150 iterations, 2.30 ms per solve before, 2.05 here.)
+// the tiles that are already in shared memory.  (ms per solve of 150 iterations
+// and 16 checks, check as separate launches / here: n = 61 1.46 / 1.31, n = 401
+// 2.01 / 1.85, n = 2000 3.17 / 2.84, n = 3000 with a CSR Q 3.91 / 3.72.)
 __device__ void res_check(const ResCheck& k, const ResArgs& a, unsigned char* sm, const DevState* cur, ResWs& ws,
                           uint32_t rank, uint32_t C) {
   __shared__ double s_red[kMaxRed][kThreads / 32];
@@ -618,8 +618,9 @@ __device__ __forceinline__ void res_sum(int n, F f, double (*s_red)[kThreads / 3
 // full and takes the sums itself, so only the products need the cluster) and
 // power_two_pass_A (kTwoPass: the norm folded into the first product and the
 // sums taken by the second product's tiles).  out[0] = lambda, out[1] =
-// iterations run.  (B200, ms per estimate before / here: n = 400 1.9 / 1.1,
-// n = 800 8.2 / 2.5, n = 2000 8.2 / 2.6, n = 3000 16.5 / 5.5.)
+// iterations run.  (B200, ms per estimate in those kernels / here: n = 61 0.76 /
+// 0.53, n = 401 1.93 / 1.04, n = 803 11.1 / 2.8, n = 2000 7.3 / 2.8, n = 3000
+// 14.0 / 5.8.)
 struct ResPower {
   double *z, *z2;         // iterates in global memory (z: the start vector)
   const double* nz2;      // kTwoPass: |z|^2 of the start vector
@@ -790,16 +791,18 @@ bool cluster_fits(int device, K kernel, int C) {
 // The cluster size for the context's problem and the slot offsets of its plans'
 // tiles in their CTA's shared memory (TileRun.soff).  c->res.ctas is 0 when the
 // problem does not fit the largest cluster or a side has a row longer than a
-// tile.  The smallest cluster is taken that holds it with at most one tile per
-// warp (or 16 CTAs).  More CTAs only add barriers to the same chains, and the
+// tile (full copies of the gathered vectors alone limit n + m to about 25,000).
+// The smallest cluster is taken that holds it with at most one tile of a side
+// per warp (or 16 CTAs).  More CTAs only add barriers to the same chains, and the
 // other SMs serve other contexts (measured on B200, us per iteration on 1 / 2 /
-// 4 / 8 / 16 CTAs: n = 61 5.3 / 6.3 / 6.2 / 6.3 / 6.7, n = 400 7.6 / 8.3 / 8.6 /
-// 8.8 / 9.3).  With fewer than one warp per tile a warp works on
-// one tile after another, and a problem of few nonzeros per row has many tiles
-// in little memory (ms per 150-iteration solve in the smallest cluster that
-// holds it / with this rule / on separate launches: n = 3000, 2 nonzeros per row,
-// cones of 33 3.77 / 2.00 / 2.77; n = 6000, cones of 3 3.06 / 1.98 / 2.85; n =
-// 3000, diagonal Q, cones of 33 5.97 / 3.92 / 5.10).
+// 4 / 8 / 16 CTAs: n = 61 3.2 / 4.3 / 4.2 / 4.4 / 4.2, n = 401 5.7 / 6.1 / 6.4 /
+// 6.7 / 7.1).  With more tiles than warps a warp works on one after another, and
+// a problem of few nonzeros per row has many tiles in little memory (us per
+// iteration in the smallest cluster that holds it / with this rule / on the
+// engine: n = 3000, 2 nonzeros per row, cones of 33 13.7 / 6.3 / 10.4; n = 6000,
+// cones of 3 11.1 / 6.8 / 10.6; n = 3000, diagonal Q, cones of 33 27.0 / 14.5 /
+// 18.6; the other way n = 1000 in cones of 65, 22 tiles with a barrier for their
+// split cones, 7.6 / 9.0 / 21.1).
 void resident_plan(Ctx* c) {
   c->res = ResidentShape();
   ResidentShape r;

@@ -82,8 +82,8 @@ def test_each_schedule_runs_its_kernels(n, launches):
 @pytest.mark.parametrize("n,dim,diag_q", [(3000, 33, False), (6000, 3, False), (1500, 33, True)])
 def test_a_sparse_small_problem_is_not_slower_on_the_automatic_schedule(n, dim, diag_q):
     """Two nonzeros per row: many tiles in little memory.  A cluster just large
-    enough to hold them left each warp several tiles in a row and took 1.2 to
-    1.6 times the engine's iteration; with one tile per warp it takes 0.6 to
+    enough to hold them leaves each warp several tiles in a row and takes 1.05
+    to 1.6 times the engine's iteration; with one tile per warp it takes 0.6 to
     0.75 times (best of 9 batches each, in turn)."""
     from hprsocp_b200 import Context
     rng = np.random.default_rng(n + dim)
